@@ -55,10 +55,11 @@
 // polynomial on the FMA pipe, to relieve the special-function unit, was measured slower here.)
 //
 // Formulas: as attention_mma.cu (reference: crates/quantinfer-runtime/src/attention.rs:105-135).
-// No load uses cluster multicast. Every mbarrier wait is bounded; on expiry the kernel sets
-// kStatusWaitTimeout and its roles leave their loops, tensor memory is freed and it returns.
+// No load uses cluster multicast. Every mbarrier wait is bounded in time; when one runs out the kernel sets
+// kStatusWaitTimeout, its roles leave their loops and meet, tensor memory is freed and it returns.
 #include "common.cuh"
 #include "attention_frag.cuh"
+#include "mbarrier.cuh"
 
 #include <cuda.h>
 #include <math.h>
@@ -66,6 +67,7 @@
 namespace {
 
 using qi_attn::smem_u32;
+using namespace qi_mbar;
 
 constexpr int BM = 128;          // query rows per CTA
 constexpr int BN = 64;           // keys per tile
@@ -75,34 +77,8 @@ constexpr int kQBytes = 2 * kHalfBytes;           // 32 KB
 constexpr int kKVHalfBytes = BN * 128;            // K or V: 64 keys x 128 bytes, one 64-column half
 constexpr int kKVBytes = 2 * kKVHalfBytes;        // 16 KB
 constexpr int kMaxTableEntries = 2048;
-constexpr uint32_t kSpinLimit = 1u << 22;   // polls of a barrier before a role gives up (each poll may itself wait a little)
 constexpr float kRescaleStep = 8.f;   // the exponent's reference follows the maximum when that has grown by more (base 2)
 
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    for (uint32_t i = 0; i < kSpinLimit; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((i & 1023u) == 1023u && *abort_flag) return false;
-    }
-    return false;
-}
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
@@ -357,13 +333,6 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     qi::pdl_wait();
     QI_TL_WAKE();
 
-    auto give_up = [&]() {
-        if (!*abort_flag) {
-            *abort_flag = 1;
-            if (status) atomicOr(status, qi::kStatusWaitTimeout);
-        }
-    };
-
     if (warp == 4) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
@@ -372,7 +341,6 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             tma_load_2d(q_s + kHalfBytes, &map_q, bars + B::q_full, h * D + 64, q0);
             // K of tile j + 1 goes out before V of tile j: a K slot is free as soon as its S has been
             // computed, a V slot only after P.V, one softmax later.
-            int issued_k = 0, issued_v = 0;
             auto load_tile = [&](int j, bool is_v) -> bool {
                 const int s = j % kStages;
                 const uint32_t empty = bars + (is_v ? B::v_empty : B::k_empty) + 8 * s;
@@ -398,25 +366,14 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                 return true;
             };
             bool ok = n_tiles == 0 || load_tile(0, false);
-            if (ok && n_tiles > 0) issued_k = 1;
             for (int j = 0; j < n_tiles && ok; ++j) {
                 if (j + 1 < n_tiles) {
                     ok = load_tile(j + 1, false);
                     if (!ok) break;
-                    issued_k = j + 2;
                 }
                 ok = load_tile(j, true);
-                if (ok) issued_v = j + 1;
             }
-            if (!ok) give_up();
-            if (*abort_flag) {   // copies in flight write into this CTA's shared memory: wait (bounded) for them
-                for (int j = max(issued_k - kStages, 0); j < issued_k; ++j)
-                    for (uint32_t t = 0; t < (1u << 20); ++t)
-                        if (mbar_try_wait(bars + B::k_full + 8 * (j % kStages), ((uint32_t)j / kStages) & 1u)) break;
-                for (int j = max(issued_v - kStages, 0); j < issued_v; ++j)
-                    for (uint32_t t = 0; t < (1u << 20); ++t)
-                        if (mbar_try_wait(bars + B::v_full + 8 * (j % kStages), ((uint32_t)j / kStages) & 1u)) break;
-            }
+            if (!ok) give_up(abort_flag, status);
         }
     } else if (warp == 5) {
         // ---------------- MMA issuer ----------------
@@ -462,7 +419,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
                 umma_commit(bars + B::v_empty + 8 * s);
                 umma_commit(bars + B::p_free + 8 * pb);
             }
-            if (!ok) give_up();
+            if (!ok) give_up(abort_flag, status);
         }
     } else {
         // ---------------- softmax threads: one query row each ----------------
@@ -472,10 +429,11 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
         float m = -INFINITY, l = 0.f;
         bool ok = true;
+        if (threadIdx.x == 0 && failed_before(status)) give_up(abort_flag, status);
         for (int j = 0; j < n_tiles && ok; ++j) {
             const uint32_t u = (uint32_t)j;
             const int t0 = tile_start(j);
-            if (!mbar_wait(bars + B::s_full, u & 1u, abort_flag)) { ok = false; break; }
+            if (!mbar_wait_warp(bars + B::s_full, u & 1u, abort_flag)) { ok = false; break; }
             tc_fence_after();
             int c_hi = min(min(pos, hi - 1) - t0 + 1, BN);
             int c_lo = max(max(lo, window > 0 ? pos - window + 1 : 0), chunk > 0 ? pos / chunk * chunk : 0) - t0;
@@ -533,7 +491,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             const bool moves = !fresh && m_top - m > kRescaleStep;
             if (__any_sync(0xffffffffu, moves)) {
                 // every product into O so far has finished: the one of tile j - 1 arrives on its buffer's barrier
-                if (!mbar_wait(bars + B::p_free + 8 * ((u - 1) & 1u), ((u - 1) >> 1) & 1u, abort_flag)) { ok = false; break; }
+                if (!mbar_wait_warp(bars + B::p_free + 8 * ((u - 1) & 1u), ((u - 1) >> 1) & 1u, abort_flag)) { ok = false; break; }
                 tc_fence_after();
                 const float f = moves ? ex2(m - m_top) : 1.f;
 #pragma unroll 1
@@ -551,7 +509,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             }
             if (fresh || moves) m = m_top;
             const float ms = (m == -INFINITY) ? 0.f : m;
-            if (u > 1 && !mbar_wait(bars + B::p_free + 8 * (u & 1u), ((u >> 1) & 1u) ^ 1u, abort_flag)) { ok = false; break; }   // P.V of tile j - 2 has read this buffer
+            if (u > 1 && !mbar_wait_warp(bars + B::p_free + 8 * (u & 1u), ((u >> 1) & 1u) ^ 1u, abort_flag)) { ok = false; break; }   // P.V of tile j - 2 has read this buffer
             uint32_t pk[BN / 2];
             const float sum = interior ? row_weights<false>(sv, pk, sc, ms - shift, 0, BN)
                                        : row_weights<true>(sv, pk, sc, ms - shift, c_lo, c_hi);
@@ -565,9 +523,9 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         // the accumulator, once the last product has finished: normalise and store
         if (ok && n_tiles > 0) {
             const uint32_t last = (uint32_t)(n_tiles - 1);
-            ok = mbar_wait(bars + B::p_free + 8 * (last & 1u), (last >> 1) & 1u, abort_flag);
+            ok = mbar_wait_warp(bars + B::p_free + 8 * (last & 1u), (last >> 1) & 1u, abort_flag);
         }
-        if (!ok && lane == 0) give_up();
+        if (!ok && lane == 0) give_up(abort_flag, status);
         if (ok && n_ranges > 1) {
             tc_fence_after();
             const size_t part = ((size_t)(q0 + row) * nq + h) * n_ranges + blockIdx.z;
@@ -623,8 +581,10 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             }
         }
     }
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
+    if (*abort_flag) settle_in_flight();
     QI_TL_END(32);
     if (warp == 5) tmem_dealloc(tmem_base, 256);
 }

@@ -12,41 +12,22 @@
 // finite (the pool is zeroed once and only finite values are written) and their
 // scores are masked, so they contribute exactly zero.
 //
-// No load uses cluster multicast. Every mbarrier wait is bounded; when a bound
-// runs out the kernel sets kStatusWaitTimeout and leaves.
+// No load uses cluster multicast. Every mbarrier wait is bounded in time; when one
+// runs out its warp sets kStatusWaitTimeout and leaves (a barrier of the block waits for the warps that are left).
 #include "attention_frag.cuh"
 #include "attention_noalloc.h"
+#include "mbarrier.cuh"
 
 #include <cuda.h>
 
 namespace {
 
 using namespace qi_attn;
+using namespace qi_mbar;
 
 constexpr int kTileKeys = 64;
-constexpr uint32_t kSpinLimit = 1u << 21;
 constexpr int kMaxTableEntries = 2048;   // block table entries one CTA keeps in shared memory
 
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < kSpinLimit; ++i)
-        if (mbar_try_wait(bar, parity)) return true;
-    return false;
-}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -166,13 +147,13 @@ attention_prefill_tma_kernel(const __grid_constant__ CUtensorMap map_q, const __
     const int row_pos[2] = {pos0 + warp * 16 + g, pos0 + warp * 16 + g + 8};
     const int warp_max_pos = pos0 + warp * 16 + 15, warp_min_pos = pos0 + warp * 16;
     const bool warp_active = warp * 16 < rows_valid;
-    bool ok = mbar_wait(q_bar, 0);
+    bool ok = mbar_wait_warp(q_bar, 0);
     if (ok) load_q_frags<D, TmaSwizzle<kPrefillRows>>(qa, q_s, warp * 16, lane);
 
     for (int i = 0; i < n_tiles && ok; ++i) {
         const int stage = i % kPrefillStages;
         const int t0 = t_begin + i * kTileKeys;
-        ok = mbar_wait(full_bar(stage), (uint32_t)(i / kPrefillStages) & 1u);
+        ok = mbar_wait_warp(full_bar(stage), (uint32_t)(i / kPrefillStages) & 1u);
         if (!ok) break;
         if (warp_active && t0 <= warp_max_pos) {
             const uint32_t k_s = kv_s + stage * 2 * kTileBytes, v_s = k_s + kTileBytes;
@@ -478,7 +459,7 @@ attention_decode_tma_kernel(const qi::bf16* __restrict__ q, qi::bf16* __restrict
     for (int i = 0; i < n_tiles; ++i) {
         const int stage = i % kDecodeStages;
         const int t0 = t_begin + i * kTileKeys;
-        ok = mbar_wait(full_bar(stage), (uint32_t)(i / kDecodeStages) & 1u);
+        ok = mbar_wait_warp(full_bar(stage), (uint32_t)(i / kDecodeStages) & 1u);
         if (!ok) break;
         if (i == 0) QI_TL_DATA();
         if (owns_new && i == n_tiles - 1) {

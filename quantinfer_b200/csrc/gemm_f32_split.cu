@@ -125,34 +125,22 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    auto give_up = [&]() {
-        if (!*abort_flag) {
-            *abort_flag = 1;
-            if (status) atomicOr(status, qi::kStatusWaitTimeout);
-        }
-    };
-
     if (warp == 0) {
         // ---------------- the tokens' parts ----------------
         if (lane == 0) {
             for (int c = 2; c < kAhead && c < chunks; ++c) prefetch_2d(&map_w, (chunk0 + c) * BK, n0);     // (the first two are read at once)
             qi::pdl_wait();
-            int c = 0;
-            for (; c < chunks; ++c) {
+            for (int c = 0; c < chunks; ++c) {
                 const int s = c & 1;
                 if (c + kAhead < chunks) prefetch_2d(&map_w, (chunk0 + c + kAhead) * BK, n0);
                 if (!mbar_wait(empty(s), ((uint32_t)(c >> 1) & 1u) ^ 1u, abort_flag, status)) {
-                    give_up();
+                    give_up(abort_flag, status);
                     break;
                 }
                 mbar_expect_tx(b_full(s), 3u * (uint32_t)width * BK * 2);
                 for (int p = 0; p < 3; ++p)
                     tma_load_2d(b_tile(s) + p * kTileBytes, &map_x, b_full(s), (chunk0 + c) * BK, p * M + t0);
             }
-            if (*abort_flag)      // copies in flight write into shared memory: wait (bounded) for the last ones
-                for (int i = max(c - 2, 0); i < c; ++i)
-                    for (uint32_t n = 0; n < (1u << 20); ++n)
-                        if (mbar_try_wait(b_full(i & 1), (uint32_t)(i >> 1) & 1u)) break;
         }
     } else if (warp == 1) {
         // ---------------- MMA ----------------
@@ -164,7 +152,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 const uint32_t parity = (uint32_t)(c >> 1) & 1u;
                 if (!mbar_wait(acc_empty(s), parity ^ 1u, abort_flag, status) || !mbar_wait(b_full(s), parity, abort_flag, status) ||
                     !mbar_wait(a_full(s), parity, abort_flag, status)) {
-                    give_up();
+                    give_up(abort_flag, status);
                     break;
                 }
                 tc_fence_after();
@@ -192,10 +180,11 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             for (int i = 0; i < 16; ++i) acc[g][i] = 0.f;
         bool ok = true;
         qi::pdl_wait();           // (every bounded wait counts from the end of the kernel before)
+        if (threadIdx.x == 64 && failed_before(status)) give_up(abort_flag, status);
         for (int c = 0; c < chunks; ++c) {
             const int s = c & 1;
-            if (!mbar_wait(acc_full(s), (uint32_t)(c >> 1) & 1u, abort_flag, status)) {
-                if (lane == 0) give_up();
+            if (!mbar_wait_warp(acc_full(s), (uint32_t)(c >> 1) & 1u, abort_flag, status)) {
+                if (lane == 0) give_up(abort_flag, status);
                 ok = false;
                 break;
             }
@@ -268,8 +257,8 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         qi::pdl_wait();
         auto chunk = [&](int c, float4 (&v)[8]) -> bool {
             const int s = c & 1;
-            if (!mbar_wait(empty(s), ((uint32_t)(c >> 1) & 1u) ^ 1u, abort_flag, status)) {
-                if (lane == 0) give_up();
+            if (!mbar_wait_warp(empty(s), ((uint32_t)(c >> 1) & 1u) ^ 1u, abort_flag, status)) {
+                if (lane == 0) give_up(abort_flag, status);
                 return false;
             }
 #pragma unroll
@@ -299,8 +288,10 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         }
         asm volatile("bar.sync 1, 512;" ::: "memory");
     }
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
+    if (*abort_flag) settle_in_flight();
     if (warp == 1) tmem_dealloc(tmem_base, 256);
 }
 

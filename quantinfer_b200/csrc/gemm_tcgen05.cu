@@ -23,11 +23,14 @@
 //              accumulator
 //   warps 2-5  read the accumulator from tensor memory (tcgen05.ld, 32 lanes x
 //              32 columns per warp) and store it
-// No load uses cluster multicast. Every mbarrier wait is bounded: when a bound
-// runs out the thread sets kStatusWaitTimeout in the status word and an abort
-// flag in shared memory, all roles leave their loops, the producer waits (with
-// a bound) for the copies it still has in flight, tensor memory is freed and
-// the kernel returns.
+// No load uses cluster multicast. Every mbarrier wait is bounded in time: when
+// one runs out the thread sets kStatusWaitTimeout in the status word and an abort
+// flag in shared memory, all roles leave their loops and meet, the block waits a
+// while for what it still has in flight, tensor memory is freed and the kernel
+// returns. A launch that finds the bit set leaves at its first wait that is not
+// fulfilled at once. (tcgen05.alloc and the barriers of a block or a cluster have
+// no bound of their own: the first waits only for blocks that end, the others
+// for roles whose waits do.)
 //
 // K must be a multiple of 8 (TMA wants row strides of whole 16 bytes); rows of
 // A, B and K beyond the tensors are zero-filled by TMA and masked at the store.
@@ -267,13 +270,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // this one: the producer fetches the first weight tiles before it waits for that kernel, the
     // epilogue warps wait before they write, and the MMA warp follows the producer's barriers.
 
-    auto give_up = [&]() {
-        if (!*abort_flag) {
-            *abort_flag = 1;
-            if (status) atomicOr(status, qi::kStatusWaitTimeout);
-        }
-    };
-
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
@@ -314,7 +310,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         continue;
                     }
                     if (!mbar_wait(empty_bar(s), ((it / STAGES) & 1u) ^ 1u, abort_flag, status)) {
-                        give_up();
+                        give_up(abort_flag, status);
                         ok = false;
                         break;
                     }
@@ -323,14 +319,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     else tma_load_2d(a_dst, &map_a, full_bar(s), k0, tile_a * BM);
                     tma_load_2d(a_dst + L::kABytes, &map_b, full_bar(s), k0, tile_b * BN);
                 }
-            }
-            if (*abort_flag) {
-                // Copies still in flight write into this CTA's shared memory: wait (bounded) for the
-                // stages armed last before the CTA may exit.
-                const uint32_t first = it > (uint32_t)STAGES ? it - STAGES : 0u;
-                for (uint32_t i = first; i < it; ++i)
-                    for (uint32_t t = 0; t < (1u << 20); ++t)
-                        if (mbar_try_wait(full_bar(i % STAGES), (i / STAGES) & 1u)) break;
             }
         }
     } else if (warp == 1) {
@@ -349,7 +337,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 const int acc = j & 1;
                 // the epilogue must have drained this accumulator (first use of each passes at once)
                 if (!mbar_wait(acc_empty_bar(acc), (((uint32_t)j >> 1) & 1u) ^ 1u, abort_flag, status)) {
-                    give_up();
+                    give_up(abort_flag, status);
                     break;
                 }
                 tc_fence_after();
@@ -357,7 +345,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 for (int i = 0; i < n_kb; ++i, ++it) {
                     const int s = it % STAGES;
                     if (!mbar_wait(full_bar(s), (it / STAGES) & 1u, abort_flag, status)) {
-                        give_up();
+                        give_up(abort_flag, status);
                         ok = false;
                         break;
                     }
@@ -380,14 +368,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         // ---------------- epilogue (warps 2..5) ----------------
         const int quarter = warp & 3;   // the 32 TMEM lanes this warp may read
         qi::pdl_wait();                 // the output buffer may still be read by the kernel before
+        if (threadIdx.x == 64 && failed_before(status)) give_up(abort_flag, status);
         int j = 0;
         for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++j) {
             const int tile_a = tile % tiles_a, tile_b = (tile / tiles_a) % tiles_b, split = tile / (tiles_a * tiles_b);
             const int kb_begin = split * kb_per_split;
             const int n_kb = max(min(kb_total, kb_begin + kb_per_split) - kb_begin, 0);
             const int acc = j & 1;
-            if (!mbar_wait(acc_full_bar(acc), ((uint32_t)j >> 1) & 1u, abort_flag, status)) {
-                if (lane == 0) give_up();
+            if (!mbar_wait_warp(acc_full_bar(acc), ((uint32_t)j >> 1) & 1u, abort_flag, status)) {
+                if (lane == 0) give_up(abort_flag, status);
                 break;
             }
             tc_fence_after();
@@ -512,8 +501,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
         }
     }
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
+    if (*abort_flag) settle_in_flight();
     QI_TL_END_SHARED(20 + EPI + (SWAP ? 0 : 5));
     if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
 }
@@ -587,6 +578,17 @@ __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
         ::"r"(bar) : "memory");
 }
 
+// As give_up(), in both CTAs of the pair: each reads the other's shared memory until the last MMA has run.
+__device__ __forceinline__ void give_up_pair(volatile int* abort_flag, int* status, uint32_t rank) {
+    if (*abort_flag) return;
+    give_up(abort_flag, status);
+    asm volatile(
+        "{\n\t.reg .b32 ra;\n\t"
+        "mapa.shared::cluster.u32 ra, %0, %1;\n\t"
+        "st.shared::cluster.u32 [ra], %2;\n\t}"
+        ::"r"(smem_u32(const_cast<const int*>(abort_flag))), "r"(rank ^ 1u), "r"(1) : "memory");
+}
+
 // out[M, N] = A[M, K] . B[N, K]^T in tiles of 256 x 256, one per pair of CTAs at a time; A are the
 // tokens, B the weights. EPI 0: the product, 2: the q/k/v projection's heads through `rope`.
 template <typename TOut, int EPI>
@@ -641,13 +643,6 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    auto give_up = [&]() {
-        if (!*abort_flag) {
-            *abort_flag = 1;
-            if (status) atomicOr(status, qi::kStatusWaitTimeout);
-        }
-    };
-
     if (warp == 0) {
         // ---------------- TMA producer (in both CTAs) ----------------
         if (lane == 0) {
@@ -681,7 +676,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                         continue;
                     }
                     if (!mbar_wait(empty_bar(s), ((it / STAGES) & 1u) ^ 1u, abort_flag, status)) {
-                        give_up();
+                        give_up_pair(abort_flag, status, rank);
                         ok = false;
                         break;
                     }
@@ -704,7 +699,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 int kb_begin;
                 const int n_kb = kb_range(tile, kb_begin);
                 if (!mbar_wait(acc_empty_bar(acc), (((uint32_t)j >> 1) & 1u) ^ 1u, abort_flag, status)) {
-                    give_up();
+                    give_up_pair(abort_flag, status, rank);
                     break;
                 }
                 tc_fence_after();
@@ -712,7 +707,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 for (int i = 0; i < n_kb; ++i, ++it) {
                     const int s = it % STAGES;
                     if (!mbar_wait(full_bar(s), (it / STAGES) & 1u, abort_flag, status)) {
-                        give_up();
+                        give_up_pair(abort_flag, status, rank);
                         ok = false;
                         break;
                     }
@@ -732,13 +727,14 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         // ---------------- epilogue (warps 2..5 of both CTAs): this CTA's 128 rows of the tile ----------------
         const int quarter = warp & 3;
         qi::pdl_wait();
+        if (threadIdx.x == 64 && failed_before(status)) give_up_pair(abort_flag, status, rank);
         int j = 0;
         for (int tile = pair; tile < total_tiles; tile += n_pairs, ++j) {
             const int tile_m = tile % tiles_m, tile_n = (tile / tiles_m) % tiles_n;
             TOut* obase = out + (size_t)(tile / (tiles_m * tiles_n)) * split_stride;
             const int acc = j & 1;
-            if (!mbar_wait(acc_full_bar(acc), ((uint32_t)j >> 1) & 1u, abort_flag, status)) {
-                if (lane == 0) give_up();
+            if (!mbar_wait_warp(acc_full_bar(acc), ((uint32_t)j >> 1) & 1u, abort_flag, status)) {
+                if (lane == 0) give_up_pair(abort_flag, status, rank);
                 break;
             }
             tc_fence_after();
@@ -787,8 +783,10 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             }
         }
     }
+    __syncwarp();
     tc_fence_before();
     cluster_sync_all();       // neither CTA goes before its partner is done with what it holds
+    if (*abort_flag) settle_in_flight();
     QI_TL_END(25 + EPI);
     if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
 }
@@ -906,13 +904,6 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
     WideTile t;
     auto blocks_of = [&](const WideTile& w) { return min(kb_total - w.split * kb_per_split, kb_per_split); };
 
-    auto give_up = [&]() {
-        if (!*abort_flag) {
-            *abort_flag = 1;
-            if (status) atomicOr(status, qi::kStatusWaitTimeout);
-        }
-    };
-
     if (warp == 0) {
         // ---------------- TMA producer (in both CTAs) ----------------
         if (lane == 0) {
@@ -939,7 +930,7 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
                     const int k0 = (kb0 + i) * BK;
                     if (it >= early) {
                         if (!mbar_wait(empty_bar(s), ((it / STAGES) & 1u) ^ 1u, abort_flag, status)) {
-                            give_up();
+                            give_up_pair(abort_flag, status, rank);
                             ok = false;
                             break;
                         }
@@ -948,13 +939,6 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
                     }
                     tma_load_2d_pair(dst + kPairHalfBytes, map_x, full_bar(s), k0, x_row);
                 }
-            }
-            if (*abort_flag && rank == 0) {
-                // copies in flight write into shared memory: wait (bounded) for the stages armed last
-                const uint32_t first = it > (uint32_t)STAGES ? it - STAGES : 0u;
-                for (uint32_t i = first; i < it; ++i)
-                    for (uint32_t n = 0; n < (1u << 20); ++n)
-                        if (mbar_try_wait(full_bar(i % STAGES), (i / STAGES) & 1u)) break;
             }
         }
     } else if (warp == 1) {
@@ -968,7 +952,7 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
                 const int acc = j & 1, n_kb = blocks_of(t);
                 const uint32_t idesc = make_idesc(2 * BM, t.width);
                 if (!mbar_wait(acc_empty_bar(acc), (((uint32_t)j >> 1) & 1u) ^ 1u, abort_flag, status)) {
-                    give_up();
+                    give_up_pair(abort_flag, status, rank);
                     break;
                 }
                 tc_fence_after();
@@ -976,7 +960,7 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
                 for (int i = 0; i < n_kb; ++i, ++it) {
                     const int s = it % STAGES;
                     if (!mbar_wait(full_bar(s), (it / STAGES) & 1u, abort_flag, status)) {
-                        give_up();
+                        give_up_pair(abort_flag, status, rank);
                         ok = false;
                         break;
                     }
@@ -997,11 +981,12 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
         const int quarter = warp & 3, set = (warp - 2) >> 2;       // a quarter's two warps take chunks of 32 columns in turn
         const bool odd = lane & 1;
         qi::pdl_wait();
+        if (threadIdx.x == 64 && failed_before(status)) give_up_pair(abort_flag, status, rank);
         int j = 0;
         for (int tile = pair; walk.locate(tile, t); tile += n_pairs, ++j) {
             const int acc = j & 1;
-            if (!mbar_wait(acc_full_bar(acc), ((uint32_t)j >> 1) & 1u, abort_flag, status)) {
-                if (lane == 0) give_up();
+            if (!mbar_wait_warp(acc_full_bar(acc), ((uint32_t)j >> 1) & 1u, abort_flag, status)) {
+                if (lane == 0) give_up_pair(abort_flag, status, rank);
                 break;
             }
             tc_fence_after();
@@ -1055,8 +1040,10 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
             if (lane == 0) mbar_arrive_leader(acc_empty_bar(acc));
         }
     }
+    __syncwarp();
     tc_fence_before();
     cluster_sync_all();       // neither CTA goes before its partner is done with what it holds
+    if (*abort_flag) settle_in_flight();
     QI_TL_END(30 + EPI);
     if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
 }

@@ -1,8 +1,9 @@
-// What the dense products on the 5th-generation tensor cores share: bounded mbarrier waits, TMA copies, tensor memory, the
-// MMA with its descriptors, and the host's tensor maps.
+// What the dense products on the 5th-generation tensor cores share: TMA copies, tensor memory, the MMA with its descriptors, and the
+// host's tensor maps (waits: mbarrier.cuh).
 #pragma once
 
 #include "common.cuh"
+#include "mbarrier.cuh"
 
 #include <cuda.h>
 
@@ -11,45 +12,11 @@ namespace {
 constexpr int BM = 128;       // rows of A per tile = MMA M
 constexpr int BK = 64;        // bf16 elements per k block = 128 bytes = one swizzle row
 constexpr int UMMA_K = 16;
-constexpr uint32_t kSpinLimit = 1u << 21;   // polls of try_wait before giving up (each poll may itself wait up to a few microseconds)
+
+using namespace qi_mbar;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-
-// Waits for the phase with the given parity to complete; false when the bound ran out
-// or another role already gave up.
-// A timeout that any CTA recorded in the global status word ends the waits of all others early.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          const volatile int* status) {
-    for (uint32_t i = 0; i < kSpinLimit; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((i & 1023u) == 1023u && *abort_flag) return false;
-        if ((i & 65535u) == 65535u && status && (*status & qi::kStatusWaitTimeout)) return false;
-    }
-    return false;
 }
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {

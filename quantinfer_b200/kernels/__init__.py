@@ -392,10 +392,6 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status=None) -
         raise KernelError(f"gemm: shapes do not agree: x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
     need = int(library().qi_gemm_f32_workspace(M, N, K))
     ws = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None
-    if status is None:
-        status = _gemm_status.get(x.device)
-        if status is None:
-            status = _gemm_status[x.device] = torch.zeros(1, dtype=torch.int32, device=x.device)
     _call('gemm', "gemm_f32", library().qi_gemm_f32, _ptr(x), _ptr(w), _ptr(out), M, N, K, _ptr(ws), _ptr(status), _stream())
 
 
@@ -912,9 +908,6 @@ def publish(src: torch.Tensor, host_out: torch.Tensor, n: int) -> None:
 # --------------------------------------------------------------------------
 # tensor-core matrix product (bfloat16 operands, 32-bit accumulation)
 
-_gemm_status = {}
-
-
 def gemm_bf16_supported(M: int, N: int, K: int, out_dtype) -> bool:
     """Whether `gemm_bf16` takes this problem; callers use `gemm_simt` otherwise."""
     return M > 0 and K % 8 == 0 and out_dtype in (torch.bfloat16, torch.float32)
@@ -964,10 +957,6 @@ def gemm_bf16(x: torch.Tensor, w: torch.Tensor, out, plan=None, status=None, epi
         if w.shape[1] != K or tuple(out.shape) != (M, n_out):
             raise KernelError(f"gemm: shapes do not agree: x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
     ws = torch.empty((splits, M, N), dtype=torch.float32, device=x.device) if splits > 1 else None
-    if status is None:
-        status = _gemm_status.get(x.device)
-        if status is None:
-            status = _gemm_status[x.device] = torch.zeros(1, dtype=torch.int32, device=x.device)
     _call('gemm', "gemm_bf16", library().qi_gemm_bf16_ex,
           _ptr(x), C.c_longlong(x.stride(0) if M > 1 else 0), _ptr(w), _ptr(None if partial_only else out),
                                 BF16 if partial_only else _code(out), M, N, K, int(swap), bn, splits, epi,

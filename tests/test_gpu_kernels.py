@@ -176,6 +176,57 @@ def test_gemm_f32_on_tensor_cores_numbers_without_parts():
     assert torch.equal(got[rows][:, cols], clean[rows][:, cols])
 
 
+FORMS = {   # M, N, K, plan
+    "weights on the rows": (33, 70000, 512, (1, 64, 1)), "tokens on the rows": (2300, 4096, 512, (0, 256, 1)),
+    "tokens on pairs": (1100, 8192, 512, (2, 256, 1)), "weights on pairs": (1100, 8192, 512, (2, 0, 1)),
+    "weights on pairs, K in parts": (1100, 8192, 1024, (2, 0, 2)), "three parts": (201, 4096, 1024, None),
+    "groups": (1100, 4096, 512, None), "attention": (1400, 4, 128, None)}
+
+
+@pytest.mark.parametrize("form", FORMS)
+def test_a_launch_after_a_wait_that_ran_out_leaves(form):
+    """With the bit of a wait that ran out in the status word a launch on the tensor cores leaves instead of computing (its blocks have
+    several tiles, so that roles are at every place when they learn of it) and keeps the bit; cleared, it computes."""
+    torch.manual_seed(3)
+    k, st = _k(), _status()
+    M, N, K, plan = FORMS[form]
+    if form == "attention":
+        nkv, ps, pages, first = 2, 64, -(-M // 64), list(range(0, M, k.QUERY_TILE))
+        kp, vp = (torch.randn(pages, nkv, ps, K, device=DEV).bfloat16() for _ in range(2))
+        q, got = torch.randn(M, N * K, device=DEV).bfloat16(), torch.empty(M, N * K, dtype=torch.bfloat16, device=DEV)
+
+        def run():
+            k.attention_prefill(q, got, kp, vp, I([list(range(pages))]), I([0, M]), I([0]), I([0] * len(first)), I(first), N, nkv, K, K ** -0.5, 0, st,
+                                impl="tcgen05")
+
+        keys, vals = (p.transpose(1, 2).reshape(-1, nkv, K)[:M].double().repeat_interleave(N // nkv, dim=1) for p in (kp, vp))
+        s = torch.einsum("ihd,jhd->hij", q.view(M, N, K).double(), keys) * K ** -0.5
+        s.masked_fill_(torch.ones(M, M, dtype=torch.bool, device=DEV).triu(1), float("-inf"))
+        ref = torch.einsum("hij,jhd->ihd", torch.softmax(s, dim=2), vals).reshape(M, N * K)
+    else:
+        groups = [0, 300, 300, 701, M] if form == "groups" else [0, M]
+        dtype = torch.float32 if form == "three parts" else torch.bfloat16
+        x, w = torch.randn(M, K, device=DEV).to(dtype), torch.randn(len(groups) - 1, N, K, device=DEV).to(dtype)
+        got = torch.empty(M, N, dtype=dtype, device=DEV)
+
+        def run():
+            if form == "three parts":
+                k.gemm_f32(x, w[0], got, status=st)
+            elif form == "groups":
+                k.gemm_bf16_grouped(x, w, got, I(groups), st)
+            else:
+                k.gemm_bf16(x, w[0], got, plan=plan, status=st)
+
+        ref = torch.cat([x[a:b].double() @ w[g].double().T for g, (a, b) in enumerate(zip(groups, groups[1:]))])
+    st.fill_(k.STATUS_WAIT_TIMEOUT)
+    run()
+    assert st.item() == k.STATUS_WAIT_TIMEOUT
+    st.zero_()
+    run()
+    # half a unit of 2^-8 of the largest value; the attention's weights are rounded to bfloat16 too
+    assert st.item() == 0 and float((got.double() - ref).abs().max()) <= float(ref.abs().max()) * 2.0 ** -8
+
+
 @pytest.mark.parametrize("rows, N, K", [
     ([1], 2, 8), ([32, 33, 0, 31], 256, 64), ([190, 0, 256, 257, 5], 384, 136), ([513, 1, 700], 130, 1032), ([0, 0, 0, 2305], 254, 72),
     ([7] * 150, 512, 264), ([0, 0], 64, 64),
