@@ -590,7 +590,8 @@ __device__ __forceinline__ void give_up_pair(volatile int* abort_flag, int* stat
 }
 
 // out[M, N] = A[M, K] . B[N, K]^T in tiles of 256 x 256, one per pair of CTAs at a time; A are the
-// tokens, B the weights. EPI 0: the product, 2: the q/k/v projection's heads through `rope`.
+// tokens, B the weights. EPI as in the kernel above (0: the product, 1: silu(gate) * up of column
+// pairs, 2: the q/k/v projection's heads through `rope`, 3: the clamped form of the pairs).
 template <typename TOut, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -760,25 +761,50 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 const int b0 = tile_n * TN + c0;
                 if (row >= rows_a) continue;
                 const bool full = b0 + 32 <= rows_b;
-                TOut* orow = obase + (size_t)row * ld_out + b0;
-                if (full && ((reinterpret_cast<uintptr_t>(orow) & 15u) == 0) && sizeof(TOut) == 2) {
+                if (EPI == 1 || EPI == 3) {
+                    // columns come in pairs (gate, up): half as many outputs
+                    TOut* orow = obase + (size_t)row * ld_out + (b0 >> 1);
+                    if (full && ((reinterpret_cast<uintptr_t>(orow) & 15u) == 0) && sizeof(TOut) == 2) {
 #pragma unroll
-                    for (int q = 0; q < 32; q += 8) {
-                        uint4 v;
-                        v.x = pack2(__uint_as_float(r[q + 0]), __uint_as_float(r[q + 1]));
-                        v.y = pack2(__uint_as_float(r[q + 2]), __uint_as_float(r[q + 3]));
-                        v.z = pack2(__uint_as_float(r[q + 4]), __uint_as_float(r[q + 5]));
-                        v.w = pack2(__uint_as_float(r[q + 6]), __uint_as_float(r[q + 7]));
-                        *reinterpret_cast<uint4*>(reinterpret_cast<qi::bf16*>(orow) + q) = v;
+                        for (int q0 = 0; q0 < 32; q0 += 16) {
+                            uint4 v;
+                            v.x = pack2(pair_act<EPI>(__uint_as_float(r[q0 + 0]), __uint_as_float(r[q0 + 1]), rope),
+                                        pair_act<EPI>(__uint_as_float(r[q0 + 2]), __uint_as_float(r[q0 + 3]), rope));
+                            v.y = pack2(pair_act<EPI>(__uint_as_float(r[q0 + 4]), __uint_as_float(r[q0 + 5]), rope),
+                                        pair_act<EPI>(__uint_as_float(r[q0 + 6]), __uint_as_float(r[q0 + 7]), rope));
+                            v.z = pack2(pair_act<EPI>(__uint_as_float(r[q0 + 8]), __uint_as_float(r[q0 + 9]), rope),
+                                        pair_act<EPI>(__uint_as_float(r[q0 + 10]), __uint_as_float(r[q0 + 11]), rope));
+                            v.w = pack2(pair_act<EPI>(__uint_as_float(r[q0 + 12]), __uint_as_float(r[q0 + 13]), rope),
+                                        pair_act<EPI>(__uint_as_float(r[q0 + 14]), __uint_as_float(r[q0 + 15]), rope));
+                            *reinterpret_cast<uint4*>(reinterpret_cast<qi::bf16*>(orow) + (q0 >> 1)) = v;
+                        }
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 32; q += 2)
+                            if (b0 + q + 1 < rows_b)
+                                store1<TOut>(orow + (q >> 1), pair_act<EPI>(__uint_as_float(r[q]), __uint_as_float(r[q + 1]), rope));
                     }
-                } else if (full && ((reinterpret_cast<uintptr_t>(orow) & 15u) == 0) && sizeof(TOut) == 4) {
-#pragma unroll
-                    for (int q = 0; q < 32; q += 4)
-                        *reinterpret_cast<uint4*>(reinterpret_cast<float*>(orow) + q) = make_uint4(r[q], r[q + 1], r[q + 2], r[q + 3]);
                 } else {
+                    TOut* orow = obase + (size_t)row * ld_out + b0;
+                    if (full && ((reinterpret_cast<uintptr_t>(orow) & 15u) == 0) && sizeof(TOut) == 2) {
 #pragma unroll
-                    for (int q = 0; q < 32; ++q)
-                        if (b0 + q < rows_b) store1<TOut>(orow + q, __uint_as_float(r[q]));
+                        for (int q = 0; q < 32; q += 8) {
+                            uint4 v;
+                            v.x = pack2(__uint_as_float(r[q + 0]), __uint_as_float(r[q + 1]));
+                            v.y = pack2(__uint_as_float(r[q + 2]), __uint_as_float(r[q + 3]));
+                            v.z = pack2(__uint_as_float(r[q + 4]), __uint_as_float(r[q + 5]));
+                            v.w = pack2(__uint_as_float(r[q + 6]), __uint_as_float(r[q + 7]));
+                            *reinterpret_cast<uint4*>(reinterpret_cast<qi::bf16*>(orow) + q) = v;
+                        }
+                    } else if (full && ((reinterpret_cast<uintptr_t>(orow) & 15u) == 0) && sizeof(TOut) == 4) {
+#pragma unroll
+                        for (int q = 0; q < 32; q += 4)
+                            *reinterpret_cast<uint4*>(reinterpret_cast<float*>(orow) + q) = make_uint4(r[q], r[q + 1], r[q + 2], r[q + 3]);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 32; ++q)
+                            if (b0 + q < rows_b) store1<TOut>(orow + q, __uint_as_float(r[q]));
+                    }
                 }
             }
         }
@@ -791,24 +817,25 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
 }
 
-// ------------------------------------------------------------------ weights on the rows of CTA pairs
+// ------------------------------------------------------------------ weights on the rows of CTA pairs, grouped
 //
-// A pair of CTAs computes 256 weight rows x up to 256 tokens with tcgen05.mma.cta_group::2; the tokens ride the MMA's N, whose width
-// is set for every tile: the rows are cut into ceil(rows / 256) tiles of equal width, rounded up to 32, so that 190 rows cost 192
-// columns and 516 cost 3 x 192, where tiles of 128 or 256 would cost 256 and 640 or 768. Two uses:
-//   grouped  the products of a mixture of experts in ONE launch: group e's rows of x [rows, K] (offsets[e] .. offsets[e + 1] - 1, read on
-//            the device) times its own weights w[e] [N, K]. The tile list (groups, then weight tiles, then token tiles: pairs that run
-//            together share weights in L2) is walked from the offsets, so no count crosses to the host and the step may sit in a graph.
-//   dense    one group (offsets null), K optionally in parts (partial sums in 32-bit, part s at out + s * split_stride); the first stages'
-//            weights are requested before the wait for the kernel before.
+// The products of a mixture of experts in ONE launch: group e's rows of x [rows, K] (offsets[e] .. offsets[e + 1] - 1,
+// read on the device) times its own weights w[e] [N, K]. A pair of CTAs computes 256 weight rows x up to 256 tokens
+// with tcgen05.mma.cta_group::2; the tokens ride the MMA's N, whose width is set for every tile: a group's rows
+// are cut into ceil(rows / 256) tiles of equal width, rounded up to 32, so that 190 rows cost 192 columns and 530
+// cost 3 x 192, where rows of 128 or 256 would cost 256 and 640 or 768. The tile list (groups, then
+// weight tiles, then token tiles: pairs that run together share weights in L2) is walked from the offsets, so no count
+// crosses to the host and the step may sit in a graph.
 // Bound by the L2's rate into the SMs (32 KB of weights and 128 bytes a token a k block and pair: 10 TB/s measured), by the weights' way in
 // from HBM below about 100 rows a group. Columns of a tile beyond its rows hold other rows' results and are not stored; weight rows
 // beyond N belong to the next group and are not stored either. Eight epilogue warps, two a quarter of tensor memory: with four, the
 // activation of a tile took longer than its products at K = 2,048 (139 -> 121 us there).
-// Measured against one dense launch an expert over four streams, which the grouped form replaced: gate, up and down of 16 experts
+// Measured against one dense launch an expert over four streams, which this replaced: gate, up and down of 16 experts
 // of 2,048 (2,048 hidden, 4 a token, 2,048 tokens) 405 -> 187 us; of 32 experts of 1,536 (4,096 hidden, 1,537 tokens) 420 -> 273 us,
 // where the weights alone take 187 us of HBM time.
-// Barriers, roles and bounds as in the kernel of pairs above.
+// Barriers, roles and bounds as in the kernel of pairs above, except that a CTA takes nothing (no tensor memory, no part in a barrier of the
+// pair) before the kernel ahead has ended, and lets the next one start only then. A dense form that took these early, and asked for its
+// first weights then, hung in a step of 647 tokens through sizes of 4,096 (no wait on an mbarrier ran out; which wait it was is not known).
 // The producer's rate of issue counts: a CTA's half of a tile's tokens (16, 32, ... 128 rows) is ONE copy, with a tensor map
 // for every height. As copies of 32 rows each, four a k block, the kernel ran at half the rate.
 struct WideMaps { CUtensorMap of[8]; };      // of[i]: boxes of 16 (i + 1) tokens
@@ -816,23 +843,20 @@ constexpr int kWideMaxGroups = 1024;
 constexpr int kWideSmem = kPairSmem + 4 * (kWideMaxGroups + 1) + 12;
 constexpr int kWideThreads = 320;            // producer, MMA, eight epilogue warps
 
-struct WideTile { int group, row0, rows, width, n0, split; };    // tokens row0 .. row0 + rows - 1 on `width` columns, weight rows from n0
+struct WideTile { int group, row0, rows, width, n0; };    // tokens row0 .. row0 + rows - 1 on `width` columns, weight rows from n0
 
 // Walks the tile list in ascending order.
 struct WideWalk {
     const int* off;
-    int groups, tiles_w, n_rows, splits;        // splits > 1 only with one group: the list once a part of K
-    int group = 0, base = 0;                    // the group reached and the tiles before it
+    int groups, tiles_w, n_rows;
+    int group = 0, base = 0;        // the group reached and the tiles before it
     __device__ __forceinline__ bool locate(int tile, WideTile& t) {
-        t.split = 0;
         for (; group < groups; ++group) {
             const int first = min(max(off[group], 0), n_rows);
             const int rows = min(max(off[group + 1], first), n_rows) - first;
             const int parts = (rows + 255) >> 8, n = parts * tiles_w;
-            if (tile < base + n * splits) {
-                int at = tile - base;
-                if (splits > 1) { t.split = at / n; at -= t.split * n; }
-                const int part = at % parts;
+            if (tile < base + n) {
+                const int at = tile - base, part = at % parts;
                 const int width = ((rows + parts - 1) / parts + 31) & ~31;
                 t.group = group;
                 t.row0 = first + part * width;
@@ -841,18 +865,17 @@ struct WideWalk {
                 t.n0 = (at / parts) * (2 * BM);
                 return true;
             }
-            base += n * splits;
+            base += n;
         }
         return false;
     }
 };
 
-template <typename TOut, int EPI>
+template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads)
-gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ WideMaps maps_x,
-                         TOut* __restrict__ out, const int* __restrict__ offsets, int groups, int n_rows, int N, int K,
-                         long long ld_out, int splits, int kb_per_split, long long split_stride, int* __restrict__ status,
-                         const RopeEpilogue act) {
+gemm_tcgen05_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ WideMaps maps_x,
+                            qi::bf16* __restrict__ out, const int* __restrict__ offsets, int groups, int n_rows, int N, int K,
+                            long long ld_out, int* __restrict__ status, const RopeEpilogue act) {
     extern __shared__ uint8_t smem_raw[];
     constexpr int STAGES = kPairStages;
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -867,11 +890,12 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
     auto acc_empty_bar = [&](int a) { return bars + 8u * (2 * STAGES + 2 + a); };
 
     QI_TL_BEGIN();
+    qi::pdl_wait();
     qi::pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-    const int kb_total = (K + BK - 1) / BK;
+    const int n_kb = (K + BK - 1) / BK;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -889,67 +913,46 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
         tmem_alloc_pair(smem_u32(tmem_slot), 512);
         tmem_relinquish_pair();
     }
-    if (offsets) {
-        qi::pdl_wait();       // they come from the kernel before
-        for (int i = threadIdx.x; i <= groups; i += kWideThreads) off[i] = offsets[i];
-    } else if (threadIdx.x == 0) {
-        off[0] = 0;
-        off[1] = n_rows;
-    }
+    for (int i = threadIdx.x; i <= groups; i += kWideThreads) off[i] = offsets[i];
     tc_fence_before();
     cluster_sync_all();       // both CTAs' barriers and tensor memory exist before anything crosses over
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    WideWalk walk{off, groups, (N + 2 * BM - 1) / (2 * BM), n_rows, splits};
+    WideWalk walk{off, groups, (N + 2 * BM - 1) / (2 * BM), n_rows};
     WideTile t;
-    auto blocks_of = [&](const WideTile& w) { return min(kb_total - w.split * kb_per_split, kb_per_split); };
 
     if (warp == 0) {
         // ---------------- TMA producer (in both CTAs) ----------------
         if (lane == 0) {
-            uint32_t it = 0, early = 0;
+            uint32_t it = 0;
             bool ok = true;
             for (int tile = pair; ok && walk.locate(tile, t); tile += n_pairs) {
-                const int half = t.width >> 1, n_kb = blocks_of(t), kb0 = t.split * kb_per_split;
+                const int half = t.width >> 1;
                 const CUtensorMap* map_x = &maps_x.of[(half >> 4) - 1];
                 const uint32_t bytes = 2u * (kPairHalfBytes + (uint32_t)half * BK * 2);
                 const int w_row = t.group * N + t.n0 + (int)rank * BM, x_row = t.row0 + (int)rank * half;
-                if (it == 0) {
-                    if (!offsets) {        // weights are never written on the device: the first ones need not wait for the kernel before
-                        early = (uint32_t)min(n_kb, STAGES);
-                        for (uint32_t i = 0; i < early; ++i) {
-                            if (rank == 0) mbar_expect_tx(full_bar(i), bytes);
-                            tma_load_2d_pair(base + i * kPairStageBytes, &map_w, full_bar(i), (kb0 + (int)i) * BK, w_row);
-                        }
-                    }
-                    qi::pdl_wait();
-                }
                 for (int i = 0; i < n_kb; ++i, ++it) {
                     const int s = it % STAGES;
                     const uint32_t dst = base + s * kPairStageBytes;
-                    const int k0 = (kb0 + i) * BK;
-                    if (it >= early) {
-                        if (!mbar_wait(empty_bar(s), ((it / STAGES) & 1u) ^ 1u, abort_flag, status)) {
-                            give_up_pair(abort_flag, status, rank);
-                            ok = false;
-                            break;
-                        }
-                        if (rank == 0) mbar_expect_tx(full_bar(s), bytes);
-                        tma_load_2d_pair(dst, &map_w, full_bar(s), k0, w_row);
+                    if (!mbar_wait(empty_bar(s), ((it / STAGES) & 1u) ^ 1u, abort_flag, status)) {
+                        give_up_pair(abort_flag, status, rank);
+                        ok = false;
+                        break;
                     }
-                    tma_load_2d_pair(dst + kPairHalfBytes, map_x, full_bar(s), k0, x_row);
+                    if (rank == 0) mbar_expect_tx(full_bar(s), bytes);
+                    tma_load_2d_pair(dst, &map_w, full_bar(s), i * BK, w_row);
+                    tma_load_2d_pair(dst + kPairHalfBytes, map_x, full_bar(s), i * BK, x_row);
                 }
             }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (the even CTA only) ----------------
         if (lane == 0 && rank == 0) {
-            qi::pdl_wait();
             uint32_t it = 0;
             int j = 0;
             bool ok = true;
             for (int tile = pair; ok && walk.locate(tile, t); tile += n_pairs, ++j) {
-                const int acc = j & 1, n_kb = blocks_of(t);
+                const int acc = j & 1;
                 const uint32_t idesc = make_idesc(2 * BM, t.width);
                 if (!mbar_wait(acc_empty_bar(acc), (((uint32_t)j >> 1) & 1u) ^ 1u, abort_flag, status)) {
                     give_up_pair(abort_flag, status, rank);
@@ -980,7 +983,6 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
         // ---------------- epilogue (warps 2..9 of both CTAs): this CTA's 128 weight rows of the tile ----------------
         const int quarter = warp & 3, set = (warp - 2) >> 2;       // a quarter's two warps take chunks of 32 columns in turn
         const bool odd = lane & 1;
-        qi::pdl_wait();
         if (threadIdx.x == 64 && failed_before(status)) give_up_pair(abort_flag, status, rank);
         int j = 0;
         for (int tile = pair; walk.locate(tile, t); tile += n_pairs, ++j) {
@@ -990,26 +992,13 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
                 break;
             }
             tc_fence_after();
-            const int own = t.n0 + (int)rank * BM + quarter * 32 + lane, n = own & ~1;      // a lane and its neighbour hold weight rows n, n + 1 (N is even)
+            const int n = t.n0 + (int)rank * BM + quarter * 32 + (lane & ~1);      // a lane and its neighbour hold weight rows n, n + 1 (N is even)
             const uint32_t tmem_tile = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)acc * 256u;
-            TOut* obase = out + (size_t)t.split * split_stride + (size_t)t.row0 * ld_out;
 #pragma unroll 1
             for (int c0 = 32 * set; c0 < t.width; c0 += 64) {
                 uint32_t r[32];
                 tmem_ld32(tmem_tile + (uint32_t)c0, r);
                 tmem_ld_wait();
-                if constexpr (sizeof(TOut) == 4) {
-                    TOut* o = obase + (size_t)c0 * ld_out + own;
-                    if (own < N) {
-#pragma unroll
-                        for (int q = 0; q < 32; ++q) {
-                            if (c0 + q < t.rows) store1<TOut>(o, __uint_as_float(r[q]));
-                            o += ld_out;
-                        }
-                    }
-                    __syncwarp();
-                    continue;
-                }
                 // Of two columns a lane keeps one and gives the other to its neighbour: even lanes end up
                 // with both weight rows of column q, odd lanes with those of q + 1. The values of a chunk are
                 // computed before any is stored: a branch around each one would leave nothing to hide the division behind.
@@ -1022,13 +1011,13 @@ gemm_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
                     v[q] = EPI == 0 ? pack2(lo, hi) : __float_as_uint(pair_act<EPI>(lo, hi, act));
                 }
                 const int c = c0 + (odd ? 1 : 0);
-                TOut* o = obase + (size_t)c * ld_out + (EPI == 0 ? n : n >> 1);
+                qi::bf16* o = out + (size_t)(t.row0 + c) * ld_out + (EPI == 0 ? n : n >> 1);
                 if (n < N) {
 #pragma unroll
                     for (int q = 0; q < 16; ++q) {
                         if (c + 2 * q < t.rows) {
                             if (EPI == 0) *reinterpret_cast<uint32_t*>(o) = v[q];
-                            else store1<TOut>(o, __uint_as_float(v[q]));
+                            else *o = __float2bfloat16_rn(__uint_as_float(v[q]));
                         }
                         o += 2 * ld_out;
                     }
@@ -1100,30 +1089,21 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, TOut* out, int M, 
     return qi::check_launch("gemm_bf16 (CTA pairs)");
 }
 
-template <typename TOut, int EPI>
-int launch_wide(const CUtensorMap& mw, const WideMaps& mx, TOut* out, const int* offsets, int groups, int n_rows, int N, int K,
-                long long ld, int* status, cudaStream_t stream, const RopeEpilogue& act, int splits = 1, long long split_stride = 0) {
-    auto kern = gemm_tcgen05_wide_kernel<TOut, EPI>;
+template <int EPI>
+int launch_grouped(const CUtensorMap& mw, const WideMaps& mx, qi::bf16* out, const int* offsets, int groups, int n_rows, int N, int K,
+                   long long ld, int* status, cudaStream_t stream, const RopeEpilogue& act) {
+    auto kern = gemm_tcgen05_grouped_kernel<EPI>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmem);
-        if (e != cudaSuccess) return qi::fail("gemm_bf16 (weights on pairs): cannot reserve %d bytes of shared memory: %s", kWideSmem, cudaGetErrorString(e));
+        if (e != cudaSuccess) return qi::fail("gemm_bf16_grouped: cannot reserve %d bytes of shared memory: %s", kWideSmem, cudaGetErrorString(e));
         configured = true;
     }
-    const long long parts = offsets ? (long long)n_rows / 256 + (groups < n_rows ? groups : n_rows) : (n_rows + 255LL) / 256;   // token tiles, at most
-    const long long tiles = parts * ((N + 2 * BM - 1) / (2 * BM)) * splits;
+    const long long tiles = ((long long)n_rows / 256 + (groups < n_rows ? groups : n_rows)) * ((N + 2 * BM - 1) / (2 * BM));   // at most
     const long long pairs = sm_count() / 2;
-    const int kb_total = (K + BK - 1) / BK;
     qi::launch(kern, dim3(2u * (unsigned)(tiles < pairs ? tiles : pairs)), dim3(kWideThreads), kWideSmem, stream, mw, mx, out, offsets, groups,
-               n_rows, N, K, ld, splits, (kb_total + splits - 1) / splits, split_stride, status, act);
-    return qi::check_launch("gemm_bf16 (weights on pairs)");
-}
-
-int make_wide_maps(CUtensorMap* mw, WideMaps* mx, const void* w, int w_rows, const void* x, int rows, int K, long long ldx) {
-    if (make_map(mw, w, w_rows, K, BM)) return 1;
-    for (int i = 0; i < 8; ++i)
-        if (make_map(&mx->of[i], x, rows, K, 16 * (i + 1), ldx)) return 1;
-    return 0;
+               n_rows, N, K, ld, status, act);
+    return qi::check_launch("gemm_bf16_grouped");
 }
 
 // Pipeline stages by tile width: as many as let two CTAs stay resident on an SM for the narrow
@@ -1148,8 +1128,8 @@ int launch_bn(int bn, const CUtensorMap& ma, const CUtensorMap& mb, TOut* out, i
 
 }  // namespace
 
-// The orientation (0: tokens on the 128 rows, 1: weights on the 128 rows, 2: CTA pairs, tokens on the rows,
-// or, with width 0, weights on the rows), tile width and K split `qi_gemm_bf16` uses when the caller does not say
+// The orientation (0: tokens on the 128 rows, 1: weights on the 128 rows, 2: tokens on the rows of
+// CTA pairs), tile width and K split `qi_gemm_bf16` uses when the caller does not say
 // (allow_split 0: the caller needs the whole sum in one CTA, as the fused activation does).
 //
 // Up to 64 tokens the product is a weight stream: the weights are the 128-row operand, the
@@ -1163,17 +1143,7 @@ int launch_bn(int bn, const CUtensorMap& ma, const CUtensorMap& mb, TOut* out, i
 // tiles of 128 x 256) and evens out a ragged last wave; its price grows with the tokens. The
 // constants were fitted to a sweep of all candidates over 72 to 4,096 tokens at four layer
 // shapes: the choice is within 1% of the best candidate on average, 10% at worst.
-//
-// Weights on the rows of CTA pairs (orientation 2 with width 0) count like the pairs of 256 x 256, times 0.4 + 0.6 width / 256 for the
-// width of their token tiles (the weights' half of a k block's traffic stays). They take every fused activation of more than 64
-// tokens (1.1 to 1.4 times as fast at ragged counts, equal within 1% at 2,048 and 8,001 in the step), and as plain products what
-// the count gives them from 112 tokens on; below that the K-split single tiles of 128 are up to 8% faster.
-// The step of 7 + 509 tokens through the 14B sizes: 18.7 -> 17.7 ms.
-static void plan_product(int M, int N, int K, int allow_split, bool allow_wide, int* swap, int* bn, int* splits) {
-    if (allow_wide && !allow_split && M > 64 && N % 2 == 0) {
-        *swap = 2; *bn = 0; *splits = 1;
-        return;
-    }
+extern "C" int qi_gemm_bf16_plan(int M, int N, int K, int allow_split, int* swap, int* bn, int* splits) {
     const int kb_total = (K + BK - 1) / BK;
     int sw = 1, b = 256, sp = 1;
     if (M <= 64) {
@@ -1226,28 +1196,8 @@ static void plan_product(int M, int N, int K, int allow_split, bool allow_wide, 
                 sp = s;
             }
         }
-        const long long parts = (M + 255) / 256;
-        const int width = ((int)((M + parts - 1) / parts) + 31) & ~31;
-        for (int si = 0; si < (allow_split && allow_wide && M >= 112 && N % 2 == 0 ? 8 : 0); ++si) {
-            const int s = split_choices[si];
-            const int kbs = (kb_total + s - 1) / s;
-            if (s > 1 && ((s - 1) * kbs >= kb_total || kbs < 8)) continue;
-            const long long waves = (parts * ((N + 255) / 256) * s + sms / 2 - 1) / (sms / 2);
-            double cost = (double)waves * (kbs + 12) * 0.87 * (0.4 + 0.6 * width / 256.0);
-            if (s > 1) cost += (double)s * M * N * 8.0 / 5.5e12 / 0.27e-6;
-            if (cost < best * 0.999) {
-                best = cost;
-                sw = 2;
-                b = 0;
-                sp = s;
-            }
-        }
     }
     *swap = sw; *bn = b; *splits = sp;
-}
-
-extern "C" int qi_gemm_bf16_plan(int M, int N, int K, int allow_split, int* swap, int* bn, int* splits) {
-    plan_product(M, N, K, allow_split, true, swap, bn, splits);
     return 0;
 }
 
@@ -1273,28 +1223,6 @@ extern "C" int qi_gemm_bf16_ex(const void* x, long long ldx, const void* w, void
     const int kb_total = (K + BK - 1) / BK;
     const int kb_per_split = (kb_total + splits - 1) / splits;
     QI_REQUIRE((splits - 1) * kb_per_split < kb_total, "gemm_bf16: %d splits leave one without work (K=%d)", splits, K);
-    if (swap == 2 && (epilogue || (bn == 0 && N % 2 == 0 && (splits > 1 || out_dtype == qi::kF32 || ((uintptr_t)out & 3) == 0)))) {
-        // weights on the rows of pairs of CTAs, tokens in tiles of equal width (a plain bfloat16 result leaves two numbers at a time)
-        CUtensorMap mw;
-        WideMaps mx;
-        if (make_wide_maps(&mw, &mx, w, N, x, M, K, ldx)) return 1;
-        if (splits > 1) {
-            float* ws = (float*)workspace;
-            if (int rc = launch_wide<float, 0>(mw, mx, ws, nullptr, 1, M, N, K, N, status, stream, glu, splits, (long long)M * N)) return rc;
-            if (out) {
-                const size_t n = (size_t)M * N;
-                unsigned blocks = (unsigned)((n + 255) / 256 < 148 * 8 ? (n + 255) / 256 : 148 * 8);
-                if (out_dtype == qi::kF32) qi::launch(splitk_reduce_kernel<float>, dim3(blocks), dim3(256), 0, stream, (const float*)ws, (float*)out, n, splits);
-                else qi::launch(splitk_reduce_kernel<qi::bf16>, dim3(blocks), dim3(256), 0, stream, (const float*)ws, (qi::bf16*)out, n, splits);
-                return qi::check_launch("splitk_reduce");
-            }
-            return 0;
-        }
-        if (epilogue == 1) return launch_wide<qi::bf16, 1>(mw, mx, (qi::bf16*)out, nullptr, 1, M, N, K, N / 2, status, stream, glu);
-        if (epilogue == 3) return launch_wide<qi::bf16, 3>(mw, mx, (qi::bf16*)out, nullptr, 1, M, N, K, N / 2, status, stream, glu);
-        if (out_dtype == qi::kF32) return launch_wide<float, 0>(mw, mx, (float*)out, nullptr, 1, M, N, K, N, status, stream, glu);
-        return launch_wide<qi::bf16, 0>(mw, mx, (qi::bf16*)out, nullptr, 1, M, N, K, N, status, stream, glu);
-    }
     if (swap == 2) {
         // pairs of CTAs: tokens on the rows, no K split
         CUtensorMap pa, pb;
@@ -1312,6 +1240,8 @@ extern "C" int qi_gemm_bf16_ex(const void* x, long long ldx, const void* w, void
             }
             return 0;
         }
+        if (epilogue == 1) return launch_pair<qi::bf16, 1>(pa, pb, (qi::bf16*)out, M, N, K, N / 2, status, stream);
+        if (epilogue == 3) return launch_pair<qi::bf16, 3>(pa, pb, (qi::bf16*)out, M, N, K, N / 2, status, stream, glu);
         if (out_dtype == qi::kF32) return launch_pair<float, 0>(pa, pb, (float*)out, M, N, K, N, status, stream);
         return launch_pair<qi::bf16, 0>(pa, pb, (qi::bf16*)out, M, N, K, N, status, stream);
     }
@@ -1372,13 +1302,15 @@ extern "C" int qi_gemm_bf16_grouped(const void* x, const void* w, void* out, con
     QI_REQUIRE(offsets, "gemm_bf16_grouped: the offsets are missing");
     CUtensorMap mw;
     WideMaps mx;
-    if (make_wide_maps(&mw, &mx, w, groups * N, x, rows, K, 0)) return 1;
+    if (make_map(&mw, w, groups * N, K, BM)) return 1;
+    for (int i = 0; i < 8; ++i)
+        if (make_map(&mx.of[i], x, rows, K, 16 * (i + 1))) return 1;
     RopeEpilogue act{};
     act.limit = limit; act.alpha = alpha;
     qi::bf16* o = (qi::bf16*)out;
-    if (epilogue == 1) return launch_wide<qi::bf16, 1>(mw, mx, o, offsets, groups, rows, N, K, N / 2, status, stream, act);
-    if (epilogue == 3) return launch_wide<qi::bf16, 3>(mw, mx, o, offsets, groups, rows, N, K, N / 2, status, stream, act);
-    return launch_wide<qi::bf16, 0>(mw, mx, o, offsets, groups, rows, N, K, N, status, stream, act);
+    if (epilogue == 1) return launch_grouped<1>(mw, mx, o, offsets, groups, rows, N, K, N / 2, status, stream, act);
+    if (epilogue == 3) return launch_grouped<3>(mw, mx, o, offsets, groups, rows, N, K, N / 2, status, stream, act);
+    return launch_grouped<0>(mw, mx, o, offsets, groups, rows, N, K, N, status, stream, act);
 }
 
 // The q/k/v projection of many tokens with what follows it fused into the epilogue:
@@ -1408,7 +1340,7 @@ extern "C" int qi_gemm_bf16_qkv_rope(const void* x, const void* w, int M, int K,
     QI_REQUIRE(n_ll < 2147483647LL, "gemm_bf16_qkv_rope: too many heads");
     const int N = (int)n_ll;
     int plan_mode, bn, plan_splits;
-    plan_product(M > 256 ? M : 257, N, K, 0, false, &plan_mode, &bn, &plan_splits);   // the width for operands that are not swapped
+    qi_gemm_bf16_plan(M > 256 ? M : 257, N, K, 0, &plan_mode, &bn, &plan_splits);   // the width for operands that are not swapped
     if (bn < 128) bn = 128;                                                        // a tile holds whole heads
     const int kb_total = (K + BK - 1) / BK;
     QI_REQUIRE((long long)((M + BM - 1) / BM) * ((N + bn - 1) / bn) < 2147483647LL, "gemm_bf16_qkv_rope: too many tiles");

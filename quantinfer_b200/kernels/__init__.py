@@ -916,9 +916,8 @@ def gemm_bf16_supported(M: int, N: int, K: int, out_dtype) -> bool:
 def gemm_bf16_plan(M: int, N: int, K: int, allow_split: bool = True):
     """(orientation, tile width, K splits) the library would choose; allow_split=False for a
     product whose epilogue needs the whole sum (the fused activation). Orientation 0: the tokens
-    ride the 128 rows of the tensor-core tile; 1: the weights do (few tokens); 2: tiles computed by pairs of CTAs, with
-    the tokens on the rows of 256 x 256, or, when the width is 0, with the weights on 256 rows and the tokens in tiles of equal
-    width (every fused activation of more than 64 tokens)."""
+    ride the 128 rows of the tensor-core tile; 1: the weights do (few tokens); 2: tokens on the rows
+    of tiles of 256 x 256 computed by pairs of CTAs (many tokens; the width is not read)."""
     key = (M, N, K, bool(allow_split))
     plan = _plans.get(key)
     if plan is None:

@@ -178,8 +178,7 @@ def test_gemm_f32_on_tensor_cores_numbers_without_parts():
 
 FORMS = {   # M, N, K, plan
     "weights on the rows": (33, 70000, 512, (1, 64, 1)), "tokens on the rows": (2300, 4096, 512, (0, 256, 1)),
-    "tokens on pairs": (1100, 8192, 512, (2, 256, 1)), "weights on pairs": (1100, 8192, 512, (2, 0, 1)),
-    "weights on pairs, K in parts": (1100, 8192, 1024, (2, 0, 2)), "three parts": (201, 4096, 1024, None),
+    "tokens on pairs": (1100, 8192, 512, (2, 256, 1)), "three parts": (201, 4096, 1024, None),
     "groups": (1100, 4096, 512, None), "attention": (1400, 4, 128, None)}
 
 

@@ -462,6 +462,37 @@ def _family(name, reqs, family):
     return steps, peak
 
 
+
+@pytest.mark.parametrize("tokens", [300, 388, 501, 647, 835, 1079])
+def test_feed_forwards_of_real_width_one_after_the_other(tokens):
+    """Clamped feed-forwards of a mixture's shared expert and of a dense layer at a width of 4,096, launched in a row with what adds them to the
+    stream, many times without a wait between: short products whose successors are all on the device before they have ended."""
+    from quantinfer_b200 import kernels
+    from quantinfer_b200.config.spec import ClampedGLUSpec
+    from quantinfer_b200.parts import Runtime
+    from quantinfer_b200.parts.moe import ClampedGLU
+
+    torch.manual_seed(tokens)
+    rt, W, limit, alpha = Runtime(torch.bfloat16, DEV), 4096, 7.0, 1.702
+    parts, refs = [], []
+    x = torch.randn(tokens, W, device=DEV).bfloat16()
+    for ff in (4096, 12288):
+        w = {n: (torch.randn(o, i, device=DEV) * 1.5 * i ** -0.5).bfloat16() for n, (o, i) in dict(gate=(ff, W), up=(ff, W), down=(W, ff)).items()}
+        part = ClampedGLU(ClampedGLUSpec(hidden_size=W, intermediate_size=ff, prefix="", limit=limit, alpha=alpha), rt)
+        part.load(w)
+        g, u = (x.double() @ w[n].double().T for n in ("gate", "up"))
+        g = g.clamp(max=limit)
+        parts.append(part)
+        refs.append((g * torch.sigmoid(alpha * g) * (u.clamp(-limit, limit) + 1)) @ w["down"].double().T)
+    resid = torch.zeros(tokens, W, device=DEV)
+    for _ in range(20):
+        for part in parts:
+            kernels.dyt(resid, part.forward(x))
+    ref = 20 * (refs[0] + refs[1])
+    assert int(rt.status.item()) == 0
+    # the activation and the outputs are rounded to bfloat16 (2^-9 of each value, independently): the sums' errors stay below that share
+    assert float((resid.double() - ref).norm() / ref.norm()) < 2.0 ** -8
+
 @pytest.mark.parametrize("name", list(CONFIGS))
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("family", ["whole", "tail", "portions", "mixed"])
