@@ -184,20 +184,23 @@ struct Tensor {
     int splits;
 };
 
-// y = x . W^T; the kernel is chosen as parts/linear.py chooses it.
-Tensor linear(Run& r, const QiLinear& L, const void* x, int x_dtype, int M, int out_dtype, bool keep_partials, void* out_given = nullptr) {
+// y = x . W^T; the kernel is chosen as parts/linear.py chooses it. What is handed on (the output or the partial sums) lies in `place`,
+// or in `out_given`, or among the other temporaries.
+Tensor linear(Run& r, const QiLinear& L, const void* x, int x_dtype, int M, int out_dtype, bool keep_partials, void* out_given = nullptr,
+              Arena* place = nullptr) {
     const int N = L.out_features, K = L.in_features;
+    Arena& result = place ? *place : r.arena;
     const bool tensor_core = x_dtype == qi::kBF16 && L.w_dtype == qi::kBF16 && M > 0 && K % 8 == 0;
     if (tensor_core) {
         int swap = 0, bn = 0, splits = 1;
         qi_gemm_bf16_plan(M, N, K, 1, &swap, &bn, &splits);
         const bool partial_only = keep_partials && splits > 1;
-        void* out = partial_only ? nullptr : (out_given ? out_given : r.arena.take((long long)M * N * esize(out_dtype)));
-        void* ws = splits > 1 ? r.arena.take((long long)splits * M * N * 4) : nullptr;
+        void* out = partial_only ? nullptr : (out_given ? out_given : result.take((long long)M * N * esize(out_dtype)));
+        void* ws = splits > 1 ? (partial_only ? result : r.arena).take((long long)splits * M * N * 4) : nullptr;
         r.call([&] { return qi_gemm_bf16(x, L.w, out, partial_only ? qi::kBF16 : out_dtype, M, N, K, swap, bn, splits, 0, ws, r.m->status, r.stream); });
         return partial_only ? Tensor{ws, qi::kF32, splits} : Tensor{out, out_dtype, 1};
     }
-    void* out = out_given ? out_given : r.arena.take((long long)M * N * esize(out_dtype));
+    void* out = out_given ? out_given : result.take((long long)M * N * esize(out_dtype));
     const long long bytes = x_dtype == qi::kF32 && L.w_dtype == qi::kF32 && out_dtype == qi::kF32 ? qi_gemm_f32_workspace(M, N, K) : 0;
     if (bytes > 0) {
         void* ws = r.arena.take(bytes);
@@ -398,8 +401,16 @@ void forward(Run& r, float* logits) {
     const int n = b.n_tokens, h = m.hidden, dt = m.act_dtype;
     float* resid = (float*)r.arena.take((long long)n * h * 4);
     r.call([&] { return qi_embedding(m.embedding, m.embedding_dtype, b.token_ids, resid, n, h, m.vocab, m.status, r.stream); });
-    // room for a feed-forward's output: its whole sum in the activation type or up to 16 partial sums
-    const long long delta_bytes = (long long)16 * n * h * 4;
+    // room for a feed-forward's output, as `linear` will hand it on: its whole sum or partial sums (products need up to 16)
+    long long delta_bytes = 0;
+    for (int i = 0; i < m.n_blocks; ++i) {
+        const QiLinear &D = m.blocks[i].down, &before = m.blocks[i ? i - 1 : 0].down;
+        if (i && D.w_dtype == before.w_dtype && D.out_features == before.out_features && D.in_features == before.in_features) continue;
+        Run dry = {r.m, r.b, Arena{nullptr, 0, 0, 0, true}, nullptr, 0, 0};
+        Arena room = {nullptr, 0, 0, 0, true};
+        linear(dry, D, nullptr, dt, n, dt, true, nullptr, &room);
+        if (room.peak > delta_bytes) delta_bytes = room.peak;
+    }
     void* delta_room[2] = {r.arena.take(delta_bytes), r.arena.take(delta_bytes)};
     const long long layer_base = r.arena.off;
     Tensor delta = {nullptr, dt, 1};
@@ -412,18 +423,9 @@ void forward(Run& r, float* logits) {
         Tensor a = attention(r, B, c, x);
         void* x2 = add_norm(r, resid, &a, B.norm2_gain, B.norm2_eps, nullptr, n, n);
         void* act = linear_act_mul(r, B.gate_up, x2, dt, n, B.activation);
-        // the down projection writes into this layer's place for what crosses to the next layer
-        QiLinear down = B.down;
-        const long long keep = r.arena.off;
-        Arena saved = r.arena;
-        r.arena.base = r.arena.dry ? nullptr : (uint8_t*)delta_room[i & 1];
-        r.arena.off = 0;
-        r.arena.size = delta_bytes;
-        delta = linear(r, down, act, dt, n, dt, true);
-        const long long used = r.arena.off;
-        r.arena = saved;
-        r.arena.off = keep;
-        if (used > delta_bytes) r.failed = 1;      // cannot happen: at most 16 splits, or one whole sum
+        // the down projection's result lies in this layer's place for what crosses to the next layer
+        Arena room = {(uint8_t*)delta_room[i & 1], delta_bytes, 0, 0, r.arena.dry};
+        delta = linear(r, B.down, act, dt, n, dt, true, nullptr, &room);
         have_delta = true;
     }
     if (b.n_logit_rows == 0) return;

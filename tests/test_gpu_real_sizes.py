@@ -49,6 +49,29 @@ def test_one_layer_at_8b_sizes(folder, dtype):
     assert float(diff.max()) <= tol, (diff.tolist(), float(expect.abs().max()))
 
 
+@pytest.mark.parametrize("hidden, ff", [(2048, 8192), (1024, 5120), (4096, 12288)])
+def test_float32_steps_whose_down_projection_is_cut_along_k(tmp_path, hidden, ff):
+    """Two float32 layers through the C++ driver, a prompt and single tokens, at widths whose down projection takes many parts of K (9, 12
+    and 5), against 64 bits, with the float32 bound of the test above. (Ten products in a row, each within 1.6e-6 of its result in 2-norms, as
+    gemm_f32_split.cu and gemm_simt.cu state for sums of this length, add up to 1.6e-5 of logits up to 4: 6.4e-5 at most.)"""
+    from quantinfer_b200.config import config_from_dict
+    from quantinfer_b200.engine import Engine, StepEntry
+    from quantinfer_b200.weights import write_model_folder
+
+    cfg_d = dict(CONFIG_8B_ONE_LAYER, vocab_size=1000, hidden_size=hidden, intermediate_size=ff, num_hidden_layers=2, num_attention_heads=8,
+                 num_key_value_heads=2)
+    folder = write_model_folder(tmp_path / "m", config_from_dict(cfg_d), seed=hidden)
+    ids = random_tokens(24, 1000, seed=5)
+    cfg, w = plain_load(folder, dtype=torch.float64)
+    expect = plain_forward(w, cfg, ids)
+    eng = Engine.from_folder(folder, dtype="float32", page_size=64, max_tokens=128, max_requests=1, max_seq_len=128)
+    eng.open("r")
+    got = [eng.step([StepEntry("r", ids[:20], list(range(20)))]).cpu()]
+    assert eng.model.native, "the driver takes this model"
+    got += [eng.step([StepEntry("r", [t], [0])]).cpu() for t in ids[20:]]
+    assert float((torch.cat(got).double() - expect).abs().max()) <= 1e-4
+
+
 # ---------------------------------------------------------------- the whole model, all 36 layers
 
 
