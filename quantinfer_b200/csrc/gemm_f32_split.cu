@@ -2,7 +2,8 @@
 // tensor cores.
 //
 // A 32-bit number is the sum of three bfloat16 numbers, h + m + l: each is the rounding of what the ones before it leave, the
-// remainders are exact in 32 bits, and 8 bits each make 24 (below 2^-110 the last part meets the smallest bfloat16 number, 2^-133).
+// remainders are exact in 32 bits, and 8 bits each make 24 (below 2^-110 the last part meets the smallest bfloat16 number, 2^-133: such
+// numbers keep fewer bits beside larger ones of their row, from 2^24 times as large on, and all of them in a row that holds no larger one).
 // bfloat16 products are exact in 32 bits, so
 //     x w = hh + (hm + mh) + (hl + mm + lh)        and what is left out (ml, lm, ll) is below 2^-25 of the product.
 // Six tcgen05 MMAs (kind::f16, 32-bit accumulation) over 64 k make a chunk; they start from zero, the five small terms first, so that
@@ -11,8 +12,10 @@
 // single FMAs that gemm_simt.cu computes: 5.7e-7 to 1.6e-6).
 //
 // A row's result depends on neither the number of rows nor the other rows: the cut of K depends on N and K alone. A row of x or w that
-// holds an infinity or a NaN (or a number that rounds to infinity as a bfloat16) is flagged on the way, and its results are
-// computed by the chain of FMAs instead, so such numbers come out as they do there.
+// holds an infinity, a NaN or a number that rounds to infinity as a bfloat16, or nothing from 2^-86 up beside zeros, is flagged on the way.
+// Its results, and every one whose sum here is not finite (parts of finite operands may overflow where the sum does not, and an infinite
+// h h meets infinities of both signs in the small terms), are computed by the chain of FMAs over all of K instead: they are what that
+// makes of them, bit for bit.
 //
 // A CTA computes 128 rows of w x up to 128 tokens (the tokens cut evenly, in steps of 16) over its part of K. Roles (18 warps):
 //   warp 0       TMA: the tokens' three parts, cut beforehand by split_rows_kernel (tokens are few, weights are not), and the
@@ -42,21 +45,34 @@ __device__ __forceinline__ void prefetch_2d(const CUtensorMap* map, int x, int y
     asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
 }
 
-// The three parts of two neighbours: packed pairs, the first number in the low half. `bad` turns into a NaN when one of them has no
-// such parts (its remainder is not finite).
-__device__ __forceinline__ void cut2(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l, float& bad) {
+// The three parts of two neighbours: packed pairs, the first number in the low half.
+__device__ __forceinline__ void cut2(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
     const __nv_bfloat162 hv = __floats2bfloat162_rn(a, b);
     h = *reinterpret_cast<const uint32_t*>(&hv);
     const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xffff0000u);
-    bad = fmaf(ra, 0.f, bad);
-    bad = fmaf(rb, 0.f, bad);
     const __nv_bfloat162 mv = __floats2bfloat162_rn(ra, rb);
     m = *reinterpret_cast<const uint32_t*>(&mv);
     const __nv_bfloat162 lv = __floats2bfloat162_rn(ra - __uint_as_float(m << 16), rb - __uint_as_float(m & 0xffff0000u));
     l = *reinterpret_cast<const uint32_t*>(&lv);
 }
 
-// parts [3, M, K] of x [M, K]; flags[row] = 1 when the row holds a number without parts. One block a row, K a multiple of 4.
+// The largest magnitude of a row, number by number; a NaN stays.
+__device__ __forceinline__ float largest(float top, float a, float b) {
+    float d;
+    asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(top), "f"(a), "f"(b));
+    return d;
+}
+// Whether a row with this largest magnitude goes through the chain of FMAs. (The first bound: half a step of bfloat16 below 2^128.)
+__device__ __forceinline__ bool needs_chain(float top) { return !(top < 3.3961775e38f) || (top != 0.f && top < 0x1p-86f); }
+
+__device__ __forceinline__ float chain(const float* __restrict__ x, const float* __restrict__ w, int K) {
+    float v = 0.f;
+#pragma unroll 4
+    for (int k = 0; k < K; ++k) v = fmaf(x[k], w[k], v);
+    return v;
+}
+
+// parts [3, M, K] of x [M, K]; flags[row] = 1 when the row needs the chain. One block a row, K a multiple of 4.
 __global__ void __launch_bounds__(256)
 split_rows_kernel(const float* __restrict__ x, qi::bf16* __restrict__ parts, int* __restrict__ flags, int M, int K) {
     qi::pdl_enter();
@@ -64,18 +80,19 @@ split_rows_kernel(const float* __restrict__ x, qi::bf16* __restrict__ parts, int
     const float4* src = reinterpret_cast<const float4*>(x + row * K);
     uint2* dst = reinterpret_cast<uint2*>(parts + row * K);
     const size_t part = (size_t)M * K / 4;
-    float bad = 0.f;
+    float top = 0.f;
     for (int i = threadIdx.x; i < K / 4; i += 256) {
         const float4 v = src[i];
         uint2 h, m, l;
-        cut2(v.x, v.y, h.x, m.x, l.x, bad);
-        cut2(v.z, v.w, h.y, m.y, l.y, bad);
+        cut2(v.x, v.y, h.x, m.x, l.x);
+        cut2(v.z, v.w, h.y, m.y, l.y);
+        top = largest(largest(top, v.x, v.y), v.z, v.w);
         dst[i] = h;
         dst[part + i] = m;
         dst[2 * part + i] = l;
     }
-    const int any = __syncthreads_or(bad != 0.f);
-    if (threadIdx.x == 0) flags[row] = any;
+    const int huge = __syncthreads_or(!(top < 3.3961775e38f)), some = __syncthreads_or(top != 0.f), real = __syncthreads_or(top >= 0x1p-86f);
+    if (threadIdx.x == 0) flags[row] = huge || (some && !real);
 }
 
 __global__ void __launch_bounds__(kSplitThreads)
@@ -88,7 +105,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     const uint32_t bars = base + kSplitBars;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(aligned + kSplitBars + 8 * 10);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    int* w_flags = reinterpret_cast<int*>(tmem_slot + 4);               // [128]
+    int* w_top = reinterpret_cast<int*>(tmem_slot + 4);                 // [128]: the largest magnitudes of the rows' parts (as bits, which order as the numbers do)
     auto a_full = [&](int s) { return bars + 8u * s; };
     auto b_full = [&](int s) { return bars + 8u * (2 + s); };
     auto empty = [&](int s) { return bars + 8u * (4 + s); };
@@ -115,7 +132,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (threadIdx.x < 128) w_flags[threadIdx.x] = 0;
+    if (threadIdx.x < 128) w_top[threadIdx.x] = 0;
     if (warp == 1) {
         tmem_alloc(smem_u32(tmem_slot), 256);
         tmem_relinquish();
@@ -204,35 +221,32 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty(s));
         }
-        asm volatile("bar.sync 1, 512;" ::: "memory");      // the converting warps have left their flags
+        asm volatile("bar.sync 1, 512;" ::: "memory");      // the converting warps have left their rows' magnitudes
         const int row = quarter * 32 + lane, n = n0 + row, count = 16 * (last - first), tf = t0 + 16 * first;
         // a lane looks at two tokens' flags: looked up where a value is stored, each would cost its latency in turn
         const bool x_any = (lane < count && tf + lane < M && x_flags[tf + lane]) || (lane + 32 < count && tf + lane + 32 < M && x_flags[tf + lane + 32]);
-        const bool w_bad = w_flags[row] != 0, special = __any_sync(0xffffffffu, x_any || w_bad);
+        bool again = needs_chain(__int_as_float(w_top[row]));
+        const bool w_bad = again;
+        again |= __any_sync(0xffffffffu, x_any);
         if (ok && n < N) {
 #pragma unroll
             for (int g = 0; g < 4; ++g)
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     const int t = tf + 16 * g + i;
-                    if (first + g < last && t < M) out[(size_t)t * N + n] = acc[g][i];
+                    if (first + g < last && t < M) {
+                        out[(size_t)t * N + n] = acc[g][i];
+                        again |= !(fabsf(acc[g][i]) <= 3.402823466e38f);
+                    }
                 }
         }
-        if (ok && n < N && special) {
-            // Not finite: the chain of FMAs; for a row of x over all of K in the first part (the others add nothing), for a row
-            // of w, whose other parts do not know, over this part.
+        if (ok && n < N && again) {
+            // with K in parts none of them can tell what the chain makes of all: a NaN asks for it where they are added
 #pragma unroll 1
             for (int i = 0; i < count && tf + i < M; ++i) {
-                const int t = tf + i;
-                const bool x_bad = x_flags[t] != 0;
-                if (!x_bad && !w_bad) continue;
-                const float* xr = x + (size_t)t * K;
-                const float* wr = w + (size_t)n * K;
-                const int from = x_bad ? 0 : chunk0 * BK, to = x_bad ? (blockIdx.y == 0 ? K : 0) : (chunk0 + chunks) * BK;
-                float v = 0.f;
-#pragma unroll 1
-                for (int k = from; k < to; ++k) v = fmaf(xr[k], wr[k], v);
-                out[(size_t)t * N + n] = v;
+                float* place = out + (size_t)(tf + i) * N + n;
+                if (!w_bad && !x_flags[tf + i] && fabsf(*place) <= 3.402823466e38f) continue;
+                *place = gridDim.y > 1 ? __int_as_float(0x7fffffff) : chain(x + (size_t)(tf + i) * K, w + (size_t)n * K, K);
             }
         }
     } else {
@@ -240,9 +254,9 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         const int tid = threadIdx.x - 320;
         const int k4 = (tid & 15) * 4, r0 = tid >> 4;          // this thread's 4 k of rows r0, r0 + 16, ...
         float4 ring[2][8];
-        float bad[8];
+        float top[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) bad[i] = 0.f;
+        for (int i = 0; i < 8; ++i) top[i] = 0.f;
         const float* src = w + (size_t)(n0 + r0) * K + (size_t)chunk0 * BK + k4;
         const size_t step = (size_t)16 * K;
         auto fetch = [&](int c, float4 (&v)[8]) {
@@ -264,18 +278,18 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 uint2 h, m, l;
-                cut2(v[i].x, v[i].y, h.x, m.x, l.x, bad[i]);
-                cut2(v[i].z, v[i].w, h.y, m.y, l.y, bad[i]);
+                cut2(v[i].x, v[i].y, h.x, m.x, l.x);
+                cut2(v[i].z, v[i].w, h.y, m.y, l.y);
+                top[i] = largest(largest(top[i], v[i].x, v[i].y), v[i].z, v[i].w);
                 const uint32_t dst = a_tile(s) + place + (uint32_t)i * 2048u;      // 16 rows further (the same place in their group of eight)
                 asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst), "r"(h.x), "r"(h.y) : "memory");
                 asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst + kTileBytes), "r"(m.x), "r"(m.y) : "memory");
                 asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst + 2 * kTileBytes), "r"(l.x), "r"(l.y) : "memory");
             }
             fetch(c + 2, v);
-            if (c + 1 == chunks || c + 2 == chunks) {
+            if (c + 1 == chunks) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    if (bad[i] != 0.f) w_flags[r0 + 16 * i] = 1;
+                for (int i = 0; i < 8; ++i) atomicMax(&w_top[r0 + 16 * i], __float_as_int(top[i]) & 0x7fffffff);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the MMA reads through the async proxy
             __syncwarp();
@@ -295,9 +309,10 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     if (warp == 1) tmem_dealloc(tmem_base, 256);
 }
 
-// out = the parts of K added in order.
+// out = the parts of K added in order; the chain where that is not finite.
 __global__ void __launch_bounds__(256)
-add_parts_kernel(const float4* __restrict__ parts, float4* __restrict__ out, size_t n4, int splits) {
+add_parts_kernel(const float4* __restrict__ parts, float4* __restrict__ out, size_t n4, int splits, const float* __restrict__ x,
+                 const float* __restrict__ w, int N, int K) {
     qi::pdl_enter();
     for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (size_t)gridDim.x * 256) {
         float4 s = parts[i];
@@ -305,6 +320,13 @@ add_parts_kernel(const float4* __restrict__ parts, float4* __restrict__ out, siz
         for (int k = 1; k < splits; ++k) {
             const float4 v = parts[k * n4 + i];
             s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        }
+        if (!(largest(largest(0.f, s.x, s.y), s.z, s.w) <= 3.402823466e38f)) {
+            const size_t t = i * 4 / N, n = i * 4 - t * N;          // (N is a multiple of 4: four columns of one row)
+            float* v = &s.x;
+#pragma unroll 1
+            for (int j = 0; j < 4; ++j)
+                if (!(fabsf(v[j]) <= 3.402823466e38f)) v[j] = chain(x + t * K, w + (n + j) * K, K);
         }
         out[i] = s;
     }
@@ -382,7 +404,7 @@ extern "C" int qi_gemm_f32(const float* x, const float* w, float* y, int M, int 
     if (splits > 1) {
         const size_t n4 = (size_t)M * N / 4;
         const size_t blocks = (n4 + 255) / 256;
-        qi::launch(add_parts_kernel, dim3((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), 0, stream, (const float4*)sums, (float4*)y, n4, splits);
+        qi::launch(add_parts_kernel, dim3((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), 0, stream, (const float4*)sums, (float4*)y, n4, splits, x, w, N, K);
         return qi::check_launch("add_parts");
     }
     return 0;

@@ -381,8 +381,9 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
 
 def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status=None) -> None:
     """out[M, N] = x[M, K] @ w[N, K]^T, all float32: by the FMA kernel of `gemm_simt`, or, for weights of real size, on the
-    tensor cores with every operand as the sum of three bfloat16 numbers, which hold its 24 bits (the error against 64
-    bits is no larger)."""
+    tensor cores with every operand as the sum of three bfloat16 numbers, which hold its 24 bits from 2^-110 up (the error against
+    64 bits is no larger). Results that are not finite, and those of rows with infinities, NaN or nothing above 2^-86, are the FMA
+    kernel's."""
     _req(x, "x", torch.float32, 2)
     _req(w, "w", torch.float32, 2)
     _req(out, "out", torch.float32, 2)

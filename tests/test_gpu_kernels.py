@@ -176,6 +176,45 @@ def test_gemm_f32_on_tensor_cores_numbers_without_parts():
     assert torch.equal(got[rows][:, cols], clean[rows][:, cols])
 
 
+@pytest.mark.parametrize("N, K", [(70000, 64), (2048, 2048)])      # K whole, and in parts
+def test_gemm_f32_on_tensor_cores_far_from_one(N, K):
+    """Finite operands whose products or sums leave the range of 32-bit numbers give what the chain of FMAs gives, bit for bit, and no
+    other result notices; so do rows of x or w that hold nothing above 2^-86, whose parts would lose bits. K stays far below the
+    range of tiny numbers beside larger ones: their lost bits are 2^-48 of the largest."""
+    torch.manual_seed(11)
+    k, M = _k(), 40
+    x, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    assert k.library().qi_gemm_f32_workspace(M, N, K) > 0
+    clean, got, chain = (torch.empty(M, N, device=DEV) for _ in range(3))
+    k.gemm_f32(x, w, clean)
+    # products far above the range, with remainders of both signs; near the largest number; infinite one way, then the other
+    x[3, 5], w[9, 5] = 1.00390625e25, 1.00390625e25
+    x[4, K - 1], w[10, K - 1] = 1.003e25, -1.0045e25
+    x[5, 0], w[11, 0] = 1.8446743e19, 1.8446743e19
+    x[6, 1], w[12, 1] = 1.30e19, 2.617e19
+    x[7, 2], x[7, K - 2], w[13, 2], w[13, K - 2] = 1e30, -1e30, 1e30, 1e30
+    x[8, 3], x[8, K - 3], w[14, 3], w[14, K - 3] = 1e30, -1e30, 1e8, 1e8        # 1e38 - 1e38
+    # rows of tiny numbers; tiny ones beside others
+    x[20] *= 2.0 ** -115
+    x[21] *= 2.0 ** -100
+    w[300] *= 2.0 ** -112
+    w[301] *= 2.0 ** -130
+    x[22, ::2] *= 2.0 ** -115
+    w[302, 1::2] *= 2.0 ** -115
+    k.gemm_f32(x, w, got)
+    k.gemm_simt(x, w, chain)
+    assert bool(chain[3, 9].isinf()) and bool(chain[5, 11].isfinite()) and bool(chain[8, 14].isfinite())
+    out_of_range = ~chain.isfinite()
+    assert torch.equal(got[out_of_range], chain[out_of_range]) and bool(got[~out_of_range].isfinite().all())
+    assert torch.equal(got[20:22], chain[20:22]) and torch.equal(got[:, 300:302], chain[:, 300:302])
+    # twice the chain's own bound: K roundings of 2^-24 of the sum of magnitudes
+    bound = K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)
+    assert bool(((got.double() - chain.double()).abs() <= bound)[~out_of_range].all())
+    rows = [i for i in range(M) if i not in (3, 4, 5, 6, 7, 8, 20, 21, 22)]
+    cols = [i for i in range(N) if i not in (9, 10, 11, 12, 13, 14, 300, 301, 302)]
+    assert torch.equal(got[rows][:, cols], clean[rows][:, cols])
+
+
 FORMS = {   # M, N, K, plan
     "weights on the rows": (33, 70000, 512, (1, 64, 1)), "tokens on the rows": (2300, 4096, 512, (0, 256, 1)),
     "tokens on pairs": (1100, 8192, 512, (2, 256, 1)), "three parts": (201, 4096, 1024, None),
