@@ -581,10 +581,9 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
             }
         }
     }
-    __syncwarp();
     tc_fence_before();
     __syncthreads();
-    if (*abort_flag) settle_in_flight();
+    if (warp == 5 && *abort_flag) settle_in_flight();
     QI_TL_END(32);
     if (warp == 5) tmem_dealloc(tmem_base, 256);
 }

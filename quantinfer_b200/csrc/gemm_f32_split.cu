@@ -302,10 +302,9 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         }
         asm volatile("bar.sync 1, 512;" ::: "memory");
     }
-    __syncwarp();
     tc_fence_before();
     __syncthreads();
-    if (*abort_flag) settle_in_flight();
+    if (warp == 1 && *abort_flag) settle_in_flight();
     if (warp == 1) tmem_dealloc(tmem_base, 256);
 }
 

@@ -501,10 +501,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
         }
     }
-    __syncwarp();
     tc_fence_before();
     __syncthreads();
-    if (*abort_flag) settle_in_flight();
+    if (warp == 1 && *abort_flag) settle_in_flight();
     QI_TL_END_SHARED(20 + EPI + (SWAP ? 0 : 5));
     if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
 }
@@ -809,10 +808,10 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             }
         }
     }
-    __syncwarp();
+    __syncwarp();             // (the barrier of the cluster takes whole warps)
     tc_fence_before();
     cluster_sync_all();       // neither CTA goes before its partner is done with what it holds
-    if (*abort_flag) settle_in_flight();
+    if (warp == 1 && *abort_flag) settle_in_flight();
     QI_TL_END(25 + EPI);
     if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
 }
@@ -1029,10 +1028,10 @@ gemm_tcgen05_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __g
             if (lane == 0) mbar_arrive_leader(acc_empty_bar(acc));
         }
     }
-    __syncwarp();
+    __syncwarp();             // (the barrier of the cluster takes whole warps)
     tc_fence_before();
     cluster_sync_all();       // neither CTA goes before its partner is done with what it holds
-    if (*abort_flag) settle_in_flight();
+    if (warp == 1 && *abort_flag) settle_in_flight();
     QI_TL_END(30 + EPI);
     if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
 }
