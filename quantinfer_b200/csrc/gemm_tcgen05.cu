@@ -537,8 +537,8 @@ __device__ __forceinline__ uint32_t cluster_rank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+__device__ __forceinline__ void cluster_sync_all() {      // (not .aligned: a role's one lane comes after the rest of its warp)
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 // The copy of a CTA of a pair; its bytes are reported to the barrier at the same address in the even CTA.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
@@ -808,7 +808,6 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             }
         }
     }
-    __syncwarp();             // (the barrier of the cluster takes whole warps)
     tc_fence_before();
     cluster_sync_all();       // neither CTA goes before its partner is done with what it holds
     if (warp == 1 && *abort_flag) settle_in_flight();
@@ -1028,7 +1027,6 @@ gemm_tcgen05_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __g
             if (lane == 0) mbar_arrive_leader(acc_empty_bar(acc));
         }
     }
-    __syncwarp();             // (the barrier of the cluster takes whole warps)
     tc_fence_before();
     cluster_sync_all();       // neither CTA goes before its partner is done with what it holds
     if (warp == 1 && *abort_flag) settle_in_flight();
