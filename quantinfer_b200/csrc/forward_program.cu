@@ -201,9 +201,9 @@ Tensor linear(Run& r, const QiLinear& L, const void* x, int x_dtype, int M, int 
         return partial_only ? Tensor{ws, qi::kF32, splits} : Tensor{out, out_dtype, 1};
     }
     void* out = out_given ? out_given : result.take((long long)M * N * esize(out_dtype));
-    const long long bytes = x_dtype == qi::kF32 && L.w_dtype == qi::kF32 && out_dtype == qi::kF32 ? qi_gemm_f32_workspace(M, N, K) : 0;
-    if (bytes > 0) {
-        void* ws = r.arena.take(bytes);
+    if (x_dtype == qi::kF32 && L.w_dtype == qi::kF32 && out_dtype == qi::kF32) {
+        const long long bytes = qi_gemm_f32_workspace(M, N, K);
+        void* ws = bytes > 0 ? r.arena.take(bytes) : nullptr;
         r.call([&] { return qi_gemm_f32((const float*)x, (const float*)L.w, (float*)out, M, N, K, ws, r.m->status, r.stream); });
         return Tensor{out, out_dtype, 1};
     }

@@ -358,17 +358,17 @@ extern "C" long long qi_gemm_f32_workspace(int M, int N, int K) {
     return (long long)(round256((size_t)3 * M * K * 2) + round256((size_t)M * 4) + (splits > 1 ? (size_t)splits * M * N * 4 : 0));
 }
 
-extern "C" int qi_gemm_simt(const void* x, int x_dtype, const void* w, int w_dtype, void* y, int y_dtype, int M, int N, int K,
-                            long long ldx, long long ldw, long long ldy, cudaStream_t stream);
+extern "C" int qi_gemm_f32_fma(const float* x, const float* w, float* y, int M, int N, int K, cudaStream_t stream);
 
-// y[M, N] = x[M, K] . w[N, K]^T, all float32, rows one after the other. workspace: qi_gemm_f32_workspace(M, N, K) bytes, 256-byte
+// y[M, N] = x[M, K] . w[N, K]^T, all float32, rows one after the other; w are weights, which no kernel in flight writes: their first rows are
+// read ahead of the stream's order. workspace: qi_gemm_f32_workspace(M, N, K) bytes, 256-byte
 // aligned (null where that is 0).
 extern "C" int qi_gemm_f32(const float* x, const float* w, float* y, int M, int N, int K, void* workspace, int* status,
                            cudaStream_t stream) {
     QI_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm_f32: bad sizes M=%d N=%d K=%d", M, N, K);
     if (M == 0) return 0;
     if (!workspace || qi_gemm_f32_workspace(M, N, K) == 0 || (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) & 15))
-        return qi_gemm_simt(x, qi::kF32, w, qi::kF32, y, qi::kF32, M, N, K, K, K, N, stream);
+        return qi_gemm_f32_fma(x, w, y, M, N, K, stream);
     QI_REQUIRE(((uintptr_t)workspace & 15) == 0, "gemm_f32: the workspace must be 16-byte aligned");
     qi::bf16* parts = (qi::bf16*)workspace;
     int* flags = (int*)((char*)workspace + round256((size_t)3 * M * K * 2));

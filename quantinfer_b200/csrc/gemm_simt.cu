@@ -98,8 +98,8 @@ int launch(const void* x, const void* w, void* y, int M, int N, int K, long long
 // copied by cp.async in their own layout, 32 k of every row a stage, rows padded to 36 floats: a 16-byte
 // read of 8 neighbouring rows then touches every bank once. A thread reads four k of its rows and
 // columns at a time, TM + TN 16-byte reads for 4 TM TN multiply-adds; the k chain of an element stays in
-// order. Small tiles have up to eight stages in flight. The first stages' weights, which no kernel of a step
-// writes, are requested before the wait for the kernel before this one.
+// order. Small tiles have up to eight stages in flight. With `ahead` the first stages' weights are requested before the wait
+// for the kernel before this one: for callers whose w no kernel in flight writes.
 // Measured, [201, 4096] . [24576, 4096]^T: 2,090 us with the kernel above, 1,168 us with this one (62% of the
 // FMA pipe's cycles, 72% of the issue slots); [201, 12288] . [4096, 12288]^T: 1,650 and 808 us. Packed FMAs
 // (fma.rn.f32x2) over a transposed copy were no faster (1,330 us): they take two cycles of the same pipe.
@@ -118,7 +118,7 @@ __device__ __forceinline__ void copy16(uint32_t dst, const float* src, bool real
 template <int TM, int TN>
 __global__ void __launch_bounds__(256, TM * TN >= 16 ? 2 : 3)
 gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y, int M, int N, int K,
-                long long ldx, long long ldw, long long ldy, long long sx, long long sw, long long sy) {
+                long long ldx, long long ldw, long long ldy, long long sx, long long sw, long long sy, int ahead) {
     constexpr int TILE_M = 16 * TM, TILE_N = 16 * TN, STAGES = f32_stages(TM, TN), STAGE = (TILE_M + TILE_N) * FS;
     extern __shared__ __align__(16) float f32_smem[];
     qi::pdl_launch_dependents();
@@ -140,8 +140,9 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
             copy16(base + 4u * ((it % STAGES) * STAGE + (offset + r) * FS + pc), real ? src + (size_t)(row0 + r) * ld + it * FK + pc : src, real);
         }
     };
+    if (!ahead) qi::pdl_wait();
     for (int it = 0; it < STAGES - 1 && it < steps; ++it) request(w, n0, N, ldw, TILE_N, TILE_M, it);
-    qi::pdl_wait();
+    if (ahead) qi::pdl_wait();
     for (int it = 0; it < STAGES - 1; ++it) {           // (the weights above belong to the first group)
         if (it < steps) request(x, m0, M, ldx, TILE_M, 0, it);
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -195,7 +196,7 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
 
 template <int TM, int TN>
 int launch_f32(const float* x, const float* w, float* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, int batch,
-               long long sx, long long sw, long long sy, cudaStream_t stream) {
+               long long sx, long long sw, long long sy, int ahead, cudaStream_t stream) {
     constexpr int smem = f32_stages(TM, TN) * f32_stage_bytes(TM, TN);
     static bool configured = false;
     if (!configured) {
@@ -204,7 +205,7 @@ int launch_f32(const float* x, const float* w, float* y, int M, int N, int K, lo
         configured = true;
     }
     const long long tiles = (long long)((M + 16 * TM - 1) / (16 * TM)) * ((N + 16 * TN - 1) / (16 * TN));
-    qi::launch(gemm_f32_kernel<TM, TN>, dim3((unsigned)tiles, 1, batch), dim3(256), smem, stream, x, w, y, M, N, K, ldx, ldw, ldy, sx, sw, sy);
+    qi::launch(gemm_f32_kernel<TM, TN>, dim3((unsigned)tiles, 1, batch), dim3(256), smem, stream, x, w, y, M, N, K, ldx, ldw, ldy, sx, sw, sy, ahead);
     return qi::check_launch("gemm_f32");
 }
 
@@ -233,11 +234,11 @@ bool f32_takes(const void* x, int x_dtype, const void* w, int w_dtype, int y_dty
 }
 
 int run_f32(const float* x, const float* w, float* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, int batch,
-            long long sx, long long sw, long long sy, cudaStream_t stream) {
+            long long sx, long long sw, long long sy, int ahead, cudaStream_t stream) {
     int tm = 1, tn = 2;
     f32_tile(M, N, batch, &tm, &tn);
     switch (tm * 16 + tn) {
-#define QI_F32(TM, TN) case TM * 16 + TN: return launch_f32<TM, TN>(x, w, y, M, N, K, ldx, ldw, ldy, batch, sx, sw, sy, stream);
+#define QI_F32(TM, TN) case TM * 16 + TN: return launch_f32<TM, TN>(x, w, y, M, N, K, ldx, ldw, ldy, batch, sx, sw, sy, ahead, stream);
 #define QI_F32_ROW(TM) QI_F32(TM, 2) QI_F32(TM, 4) QI_F32(TM, 8)
         QI_F32_ROW(1) QI_F32_ROW(2) QI_F32_ROW(3) QI_F32_ROW(4) QI_F32_ROW(6) QI_F32_ROW(7) QI_F32_ROW(8)
 #undef QI_F32_ROW
@@ -256,7 +257,7 @@ extern "C" int qi_gemm_simt(const void* x, int x_dtype, const void* w, int w_dty
     QI_REQUIRE((M + BM - 1) / BM <= 65535, "gemm_simt: M=%d is too large for one launch", M);
     if (M == 0) return 0;
     if (f32_takes(x, x_dtype, w, w_dtype, y_dtype, M, N, K, ldx, ldw, 0, 0))
-        return run_f32((const float*)x, (const float*)w, (float*)y, M, N, K, ldx, ldw, ldy, 1, 0, 0, 0, stream);
+        return run_f32((const float*)x, (const float*)w, (float*)y, M, N, K, ldx, ldw, ldy, 1, 0, 0, 0, 0, stream);
     QI_DISPATCH_DTYPE(x_dtype, TX, {
         QI_DISPATCH_DTYPE(w_dtype, TW, {
             QI_DISPATCH_DTYPE(y_dtype, TY, {
@@ -265,6 +266,14 @@ extern "C" int qi_gemm_simt(const void* x, int x_dtype, const void* w, int w_dty
         });
     });
     return 0;
+}
+
+// y[M, N] = x[M, K] . w[N, K]^T, all float32, rows one after the other, w's first rows read ahead of the stream's order (weights, which no
+// kernel in flight writes).
+extern "C" int qi_gemm_f32_fma(const float* x, const float* w, float* y, int M, int N, int K, cudaStream_t stream) {
+    if (M > 0 && N > 0 && K > 0 && f32_takes(x, qi::kF32, w, qi::kF32, qi::kF32, M, N, K, K, K, 0, 0))
+        return run_f32(x, w, y, M, N, K, K, K, N, 1, 0, 0, 0, 1, stream);
+    return qi_gemm_simt(x, qi::kF32, w, qi::kF32, y, qi::kF32, M, N, K, K, K, N, stream);
 }
 
 // A batch of such products in one launch: product b reads x + b * sx, w + b * sw and writes y + b * sy
@@ -279,7 +288,7 @@ extern "C" int qi_gemm_simt_batched(const void* x, int x_dtype, const void* w, i
     QI_REQUIRE((M + BM - 1) / BM <= 65535, "gemm_simt_batched: M=%d is too large for one launch", M);
     if (M == 0) return 0;
     if (f32_takes(x, x_dtype, w, w_dtype, y_dtype, M, N, K, ldx, ldw, sx, sw))
-        return run_f32((const float*)x, (const float*)w, (float*)y, M, N, K, ldx, ldw, ldy, batch, sx, sw, sy, stream);
+        return run_f32((const float*)x, (const float*)w, (float*)y, M, N, K, ldx, ldw, ldy, batch, sx, sw, sy, 0, stream);
     QI_DISPATCH_DTYPE(x_dtype, TX, {
         QI_DISPATCH_DTYPE(w_dtype, TW, {
             QI_DISPATCH_DTYPE(y_dtype, TY, {

@@ -383,7 +383,7 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status=None) -
     """out[M, N] = x[M, K] @ w[N, K]^T, all float32: by the FMA kernel of `gemm_simt`, or, for weights of real size, on the
     tensor cores with every operand as the sum of three bfloat16 numbers, which hold its 24 bits from 2^-110 up (the error against
     64 bits is no larger). Results that are not finite, and those of rows with infinities, NaN or nothing above 2^-86, are the FMA
-    kernel's."""
+    kernel's. w are weights: their first rows may be read before the library's kernels that are still in flight have ended."""
     _req(x, "x", torch.float32, 2)
     _req(w, "w", torch.float32, 2)
     _req(out, "out", torch.float32, 2)
@@ -938,7 +938,8 @@ def gemm_bf16(x: torch.Tensor, w: torch.Tensor, out, plan=None, status=None, epi
 
     epilogue="silu_mul": w's rows are (gate, up) pairs and out is [M, N / 2] =
     silu(gate) * up; "glu_clamped" with `glu` = (limit, alpha): g sigmoid(alpha g) (u + 1), g = min(gate, limit), u =
-    clamp(up, -limit, limit). x may be a block of columns of wider rows (a multiple of 8 elements apart). keep_partials=True: when the plan splits K, the float32 partial sums
+    clamp(up, -limit, limit). w are weights: their first rows may be read before the library's kernels that are still in flight have ended.
+    x may be a block of columns of wider rows (a multiple of 8 elements apart). keep_partials=True: when the plan splits K, the float32 partial sums
     [splits, M, N] are returned unreduced (and `out` is not written); else `out` is returned."""
     _cols(x, "x", torch.bfloat16)
     _req(w, "w", torch.bfloat16, 2)

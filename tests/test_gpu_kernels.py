@@ -130,6 +130,29 @@ def test_gemm_f32_keeps_the_order_of_its_sums(M, N, K):
     assert bool(((fast.double() - x.double() @ w.double().T).abs() <= bound).all())
 
 
+def test_gemm_simt_reads_what_the_kernel_before_it_wrote():
+    """Both operands may be another kernel's results: a chain of products whose second operand the launch before wrote, over buffers that
+    hold other numbers before."""
+    torch.manual_seed(2)
+    k, n = _k(), 1024
+    a = torch.randn(n, n, device=DEV) * n ** -0.5
+    steps = [torch.randn(n, n, device=DEV) * n ** -0.5 for _ in range(2)]
+    for small in (False, True):
+        x = a[:24].contiguous() if small else a
+        want, w = [], a
+        for i in range(12):
+            w = steps[i % 2].double() @ w.double().T
+            want.append(x.double() @ w.T)
+        got, bufs, w = [], [torch.full((n, n), 1e3, device=DEV) for _ in range(12)], a
+        for i in range(12):
+            k.gemm_simt(steps[i % 2], w, bufs[i])
+            got.append(torch.full((x.shape[0], n), -1e3, device=DEV))
+            k.gemm_simt(x, bufs[i], got[-1])
+            w = bufs[i]
+        # each product's error is at most K 2^-24 of the sum of magnitudes, which is about 32 times the result here; twelve in a row
+        assert max(float((g.double() - r).norm() / r.norm()) for g, r in zip(got, want)) < 12 * 32 * n * 2.0 ** -24
+
+
 @pytest.mark.parametrize("N, K", [(4096, 1024), (1028, 4096), (512, 8192), (70000, 64), (1024, 4160)])
 def test_gemm_f32_on_tensor_cores(N, K):
     """Three bfloat16 parts an operand: no further from 64 bits than the chain of single FMAs, over the edges of the token tiles; a row is the
