@@ -348,13 +348,42 @@ int parts_of_k(int N, int K) {
 
 size_t round256(size_t n) { return (n + 255) & ~(size_t)255; }
 
+// Rows of x that go through the workspace at a time: the partial sums of a long prompt would take gigabytes (8,001 rows by 24,576
+// columns in 3 parts: 2.4 GB), and eight tiles of tokens already share every tile of weights that comes from HBM.
+constexpr int kRowsAtOnce = 1024;
+
+int run_rows(const float* x, const float* w, float* y, int M, int N, int K, void* workspace, const CUtensorMap& mw, int* status, cudaStream_t stream) {
+    qi::bf16* parts = (qi::bf16*)workspace;
+    int* flags = (int*)((char*)workspace + round256((size_t)3 * M * K * 2));
+    float* sums = (float*)((char*)flags + round256((size_t)M * 4));
+    const int splits = parts_of_k(N, K), each = (K / BK + splits - 1) / splits;
+    const int tiles_t = (M + 127) / 128, width = ((M + tiles_t - 1) / tiles_t + 15) & ~15;
+    const long long tiles = (long long)((N + 127) / 128) * tiles_t;
+    QI_REQUIRE(tiles < 2147483647LL, "gemm_f32: too many tiles");
+    CUtensorMap mx;
+    if (make_map(&mx, parts, 3 * M, K, width)) return 1;
+    qi::launch(split_rows_kernel, dim3(M), dim3(256), 0, stream, x, parts, flags, M, K);
+    if (int rc = qi::check_launch("split_rows")) return rc;
+    qi::launch(gemm_f32_split_kernel, dim3((unsigned)tiles, splits), dim3(kSplitThreads), kSplitSmem, stream, mx, mw, x, w, splits > 1 ? sums : y,
+               (const int*)flags, M, N, K, width, tiles_t, each, status);
+    if (int rc = qi::check_launch("gemm_f32_split")) return rc;
+    if (splits > 1) {
+        const size_t n4 = (size_t)M * N / 4;
+        const size_t blocks = (n4 + 255) / 256;
+        qi::launch(add_parts_kernel, dim3((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), 0, stream, (const float4*)sums, (float4*)y, n4, splits, x, w, N, K);
+        return qi::check_launch("add_parts");
+    }
+    return 0;
+}
+
 }  // namespace
 
 // Bytes of workspace that qi_gemm_f32 needs for a product of these sizes; 0: it takes gemm_simt.cu's kernel, which needs none.
 // The line: below 2^22 weights (16 MB) both are a matter of latency and the FMA kernel, one launch instead of two or three, is the faster one.
 extern "C" long long qi_gemm_f32_workspace(int M, int N, int K) {
-    if (M <= 0 || N <= 0 || K <= 0 || K % BK || N % 4 || (long long)N * K < (1LL << 22) || (long long)3 * M >= 2147483647LL) return 0;
+    if (M <= 0 || N <= 0 || K <= 0 || K % BK || N % 4 || (long long)N * K < (1LL << 22)) return 0;
     const int splits = parts_of_k(N, K);
+    if (M > kRowsAtOnce) M = kRowsAtOnce;
     return (long long)(round256((size_t)3 * M * K * 2) + round256((size_t)M * 4) + (splits > 1 ? (size_t)splits * M * N * 4 : 0));
 }
 
@@ -370,15 +399,7 @@ extern "C" int qi_gemm_f32(const float* x, const float* w, float* y, int M, int 
     if (!workspace || qi_gemm_f32_workspace(M, N, K) == 0 || (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) & 15))
         return qi_gemm_f32_fma(x, w, y, M, N, K, stream);
     QI_REQUIRE(((uintptr_t)workspace & 15) == 0, "gemm_f32: the workspace must be 16-byte aligned");
-    qi::bf16* parts = (qi::bf16*)workspace;
-    int* flags = (int*)((char*)workspace + round256((size_t)3 * M * K * 2));
-    float* sums = (float*)((char*)flags + round256((size_t)M * 4));
-    const int splits = parts_of_k(N, K), each = (K / BK + splits - 1) / splits;
-    const int tiles_t = (M + 127) / 128, width = ((M + tiles_t - 1) / tiles_t + 15) & ~15;
-    const long long tiles = (long long)((N + 127) / 128) * tiles_t;
-    QI_REQUIRE(tiles < 2147483647LL, "gemm_f32: too many tiles");
-    CUtensorMap mx, mw;
-    if (make_map(&mx, parts, 3 * M, K, width)) return 1;
+    CUtensorMap mw;
     {
         EncodeTiledFn enc = get_encode();
         if (!enc) return qi::fail("gemm_f32: cuTensorMapEncodeTiled is not available from the driver");
@@ -395,16 +416,7 @@ extern "C" int qi_gemm_f32(const float* x, const float* w, float* y, int M, int 
             return qi::fail("gemm_f32: %d bytes of shared memory were refused", kSplitSmem);
         configured = true;
     }
-    qi::launch(split_rows_kernel, dim3(M), dim3(256), 0, stream, x, parts, flags, M, K);
-    if (int rc = qi::check_launch("split_rows")) return rc;
-    qi::launch(gemm_f32_split_kernel, dim3((unsigned)tiles, splits), dim3(kSplitThreads), kSplitSmem, stream, mx, mw, x, w, splits > 1 ? sums : y,
-               (const int*)flags, M, N, K, width, tiles_t, each, status);
-    if (int rc = qi::check_launch("gemm_f32_split")) return rc;
-    if (splits > 1) {
-        const size_t n4 = (size_t)M * N / 4;
-        const size_t blocks = (n4 + 255) / 256;
-        qi::launch(add_parts_kernel, dim3((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), 0, stream, (const float4*)sums, (float4*)y, n4, splits, x, w, N, K);
-        return qi::check_launch("add_parts");
-    }
+    for (int r = 0; r < M; r += kRowsAtOnce)
+        if (int rc = run_rows(x + (size_t)r * K, w, y + (size_t)r * N, M - r < kRowsAtOnce ? M - r : kRowsAtOnce, N, K, workspace, mw, status, stream)) return rc;
     return 0;
 }

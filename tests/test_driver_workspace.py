@@ -44,3 +44,9 @@ SIZES = [(2048, 8192), (1536, 8960), (1024, 5120), (896, 4864), (3072, 24576), (
 def test_every_size_has_a_workspace(lib, hidden, ff, n, dtype):
     got = _bytes(lib, hidden, ff, n, dtype)
     assert got > 0, (got, lib.qi_last_error())
+
+
+def test_long_float32_prompts_do_not_keep_partial_sums_of_every_row(lib):
+    """8,001 tokens through two layers of 4,096 x 12,288 in float32: the layer's own tensors (residual stream, q/k/v, gate and up and their
+    product, two outputs: about 2.4 GB) and a workspace that no longer grows with the tokens."""
+    assert _bytes(lib, 4096, 12288, 8001, FLOAT32, heads=32, kv=8) < 3.2e9

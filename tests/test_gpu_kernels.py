@@ -175,6 +175,23 @@ def test_gemm_f32_on_tensor_cores(N, K):
         assert torch.equal(out, whole[300 - M:])
 
 
+@pytest.mark.parametrize("M", [1023, 1025, 2100])
+def test_gemm_f32_on_tensor_cores_rows_in_passes(M):
+    """More rows than go through the workspace at a time: every row is what it is alone, with K whole and in parts, and the workspace does not grow."""
+    torch.manual_seed(M)
+    k = _k()
+    for N, K in ((70000, 64), (1028, 4096)):
+        x, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV) * 0.02
+        x[M - 1, 3] = float("inf")
+        got = torch.empty(M, N, device=DEV)
+        k.gemm_f32(x, w, got)
+        for a, b in ((0, 128), (1000, M), (M - 1, M)):
+            part = torch.empty(b - a, N, device=DEV)
+            k.gemm_f32(x[a:b].contiguous(), w, part)
+            assert torch.equal(part.nan_to_num(1e9), got[a:b].nan_to_num(1e9))
+        assert k.library().qi_gemm_f32_workspace(M, N, K) <= k.library().qi_gemm_f32_workspace(1024, N, K)
+
+
 def test_gemm_f32_on_tensor_cores_numbers_without_parts():
     """Infinities, NaN and numbers that round to infinity as a bfloat16: what the chain of FMAs makes of them, and no other row or column
     notices. Parts of K are added, so that finite results may differ in their last bits."""
