@@ -25,8 +25,8 @@
 //   warps 10-17  read w (32-bit, up to two chunks of 32 KB ahead in registers, from the L2), cut it, and write the three
 //                tiles to shared memory in the layout of the 128-byte swizzle
 // Two stages of both operands' parts fill the shared memory (192 KB). What bounds a chunk is the way of a stage from the converting
-// warps through the MMAs and back, 1.2 us for one token and 1.4 for 100: leaving out the conversion, the loads or most MMAs, one at a
-// time, saved under 10%. Waits are bounded as in gemm_tcgen05.cu.
+// warps through the MMAs and back, 1.2 us for one token and 1.4 for 100: leaving out the conversion, the loads or most MMAs (24 of
+// 70 cycles each, 0.9 us, run beside the next stage's conversion), one at a time, saved under 10%. Waits are bounded as in gemm_tcgen05.cu.
 // Measured against the chain of FMAs, one token and 201: [4096, 4096] 87 -> 37 and 270 -> 68 us; [24576, 4096] 325 -> 143 and
 // 1,166 -> 292 us; [4096, 12288] 255 -> 75 and 805 -> 154 us.
 #include "common.cuh"

@@ -508,7 +508,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
 }
 
-// Adds split-K partial sums in split order: out[i] = sum_s partial[s, i].
 // ------------------------------------------------------------------ two CTAs on one tile
 //
 // For many tokens the single-CTA kernel is bound by what its 128 x 256 tiles draw from L2 and
@@ -524,7 +523,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 //   acc_full  in each CTA: the same at the end of a tile
 //   acc_empty in the even CTA: the four epilogue warps of both CTAs arrive there
 // No load uses cluster multicast. All waits are bounded as in the kernel above; a CTA that
-// gave up is seen by its partner through the status word. Both CTAs pass a cluster barrier
+// gives up says so in its partner's shared memory too. Both CTAs pass a cluster barrier
 // before they leave, so that neither frees shared or tensor memory its partner still uses.
 
 constexpr int kPairStages = 6;
@@ -1034,6 +1033,7 @@ gemm_tcgen05_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __g
     if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
 }
 
+// Adds split-K partial sums in split order: out[i] = sum_s partial[s, i].
 template <typename TOut>
 __global__ void splitk_reduce_kernel(const float* __restrict__ partial, TOut* __restrict__ out, size_t n, int splits) {
     qi::pdl_enter();
@@ -1221,7 +1221,7 @@ extern "C" int qi_gemm_bf16_ex(const void* x, long long ldx, const void* w, void
     const int kb_per_split = (kb_total + splits - 1) / splits;
     QI_REQUIRE((splits - 1) * kb_per_split < kb_total, "gemm_bf16: %d splits leave one without work (K=%d)", splits, K);
     if (swap == 2) {
-        // pairs of CTAs: tokens on the rows, no K split
+        // pairs of CTAs: tokens on the rows (the width of a plan is not read)
         CUtensorMap pa, pb;
         if (make_map(&pa, x, M, K, BM, ldx)) return 1;
         if (make_map(&pb, w, N, K, BM)) return 1;

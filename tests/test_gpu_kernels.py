@@ -373,7 +373,7 @@ def test_attention_generic_by_pieces_and_by_elements(dtype, d, dv, window, keep)
     # pairs of CTAs on tiles of 256 x 256: one tile, ragged edges in both directions, many k blocks, more tiles than pairs
     (256, 256, 64, (2, 256, 1)), (300, 400, 136, (2, 256, 1)), (129, 130, 1032, (2, 256, 1)), (2560, 2304, 320, (2, 256, 1)),
     (512, 300, 2048, (2, 256, 3)), (700, 1100, 1600, (2, 256, 2)),      # the same with K split: partial sums, then added
-    # weights on the rows of pairs, tokens in tiles of equal width: one tile, ragged edges, several widths, K split, more tiles than pairs
+    # plans of width 0, whose width is not read (the same kernel of pairs): one tile, ragged edges, K split, more tiles than pairs
     (1, 256, 64, (2, 0, 1)), (33, 130, 136, (2, 0, 1)), (516, 520, 1032, (2, 0, 1)), (257, 2304, 320, (2, 0, 1)),
     (2305, 1026, 192, (2, 0, 1)), (65, 300, 2048, (2, 0, 3)), (700, 1100, 1600, (2, 0, 2)), (129, 9000, 520, (2, 0, 3)),
 ])
